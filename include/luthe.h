@@ -34,7 +34,10 @@
  *    ((i*2 + row)*2 + col)*N + c: GGSW of LWE-key bit i, row = decomposed GLWE
  *    component (0 mask, 1 body), col = output component.  The engine converts
  *    it to its own evaluation layout on upload (the HPU too receives its BSK
- *    pre-transformed from the host: hw/module/bsk/module/bsk_manager).
+ *    pre-transformed from the host: hw/module/bsk/module/bsk_manager), and,
+ *    where the HBM budget has room for it, to the operand form of the
+ *    tensor-core blind rotation (2.0 MB per LWE coefficient and 63 MB of
+ *    workspace; given up again when a later allocation needs the room).
  *  - LUT:  trivial GLWE, mask polynomial then body polynomial, natural order.
  */
 #ifndef LUTHE_H
@@ -137,9 +140,8 @@ int luthe_ks_pbs(luthe_ctx *ctx, const uint64_t *d_in, const uint32_t *d_lut_id,
  * Pinned host memory gives the full PCIe/C2C bandwidth.  Batches of 1024 or
  * more are copied in as two chunks (a quarter, then the rest) on a stream of
  * the context, each chunk's key switch starting once it has landed; when the
- * batch ends in a partial
- * wave that runs as its own launch, the outputs of the full waves are copied
- * back on that stream while that launch runs. */
+ * batch takes several launches, the outputs of all but the last are copied
+ * back on that stream while the last one runs. */
 int luthe_ks_pbs_host(luthe_ctx *ctx, const uint64_t *h_in, const uint32_t *h_lut_id, uint64_t *h_out,
                       size_t count);
 /* Many-LUT PBS (PBS_ML2/ML4/ML8, docs/dop.md:101-121): one blind rotation per
@@ -219,7 +221,9 @@ int luthe_server_counters(luthe_server *srv, uint64_t *rounds, uint64_t *pbs, ui
  * idle lane. */
 int luthe_server_set_batching(luthe_server *srv, uint32_t fill, uint32_t window_us);
 
-/* Blind-rotation launch shape (the HPU's batch configuration: the BSK slice
+/* Blind-rotation launch shape of batches, or remainders of batches, of at most
+ * one ciphertext per SM, and of all batches of a context without the
+ * tensor-core form (the HPU's batch configuration: the BSK slice
  * shared per batch, hw/module/pe_pbs/module/pep_sequencer/rtl/
  * pep_sequencer.sv:573-620, docs/hpu_parameters.md): ciphertexts per CTA
  * sharing one BSK slab (1 or 2) and CTAs per SM of the persistent grid;

@@ -56,12 +56,23 @@ static int check_params(const luthe_params *p)
     return LUTHE_OK;
 }
 
+static void brx_release(luthe_ctx *c);
+
 int dalloc(luthe_ctx *c, void **ptr, size_t bytes)
 {
+    // the tensor-core blind rotation's key and workspace are optional: they
+    // give way to anything else the context is asked to hold
+    if (c->used + bytes > c->budget) brx_release(c);
     if (c->used + bytes > c->budget)
         return fail(LUTHE_E_BUDGET, "HBM budget exceeded: %llu + %zu > %llu bytes", (unsigned long long)c->used,
                     bytes, (unsigned long long)c->budget);
-    CUDA_TRY(cudaMalloc(ptr, bytes));
+    cudaError_t e = cudaMalloc(ptr, bytes);
+    if (e == cudaErrorMemoryAllocation && c->ws.bsk) {
+        cudaGetLastError();
+        brx_release(c);
+        e = cudaMalloc(ptr, bytes);
+    }
+    CUDA_TRY(e);
     c->used += bytes;
     return LUTHE_OK;
 }
@@ -77,6 +88,64 @@ void drop_graphs(luthe_ctx *c)
 {
     for (auto &g : c->graphs) cudaGraphExecDestroy(g.exec);
     c->graphs.clear();
+}
+
+// ---- tensor-core blind rotation: expanded key and workspace (brx.cu)
+
+static size_t brx_bytes(const luthe_ctx *c)
+{
+    using namespace brx;
+    return (size_t)c->p.lwe_dim * STEP_BYTES + WEIGHT_BYTES + (EVAL_WORDS + PROD_WORDS + ACC_WORDS) * 8 +
+           SYNC_BYTES;
+}
+
+static void brx_release(luthe_ctx *c)
+{
+    if (!c->ws.weights) return;
+    drop_graphs(c);  // captured launches use the workspace
+    cudaFree(c->ws.weights);  // one allocation
+    c->ws = brx::Workspace{};
+    c->used -= brx_bytes(c);
+}
+
+// Allocate (first key) and fill the expanded key from the standard-domain BSK
+// on the device.  Without room for it the context works without: every batch
+// then runs the butterfly kernels.
+static int brx_prepare(luthe_ctx *c, const uint64_t *d_std)
+{
+    using namespace brx;
+    if (!c->ws.weights) {
+        const size_t bytes = brx_bytes(c);
+        int cooperative = 0;
+        CUDA_TRY(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, c->device));
+        if (!cooperative || c->used + bytes > c->budget) return LUTHE_OK;
+        uint8_t *base = nullptr;
+        if (cudaMalloc((void **)&base, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return LUTHE_OK;
+        }
+        Workspace w;
+        w.bsk = base + WEIGHT_BYTES;
+        w.eval = (uint64_t *)(w.bsk + (size_t)c->p.lwe_dim * STEP_BYTES);
+        w.prod = w.eval + EVAL_WORDS;
+        w.acc = w.prod + PROD_WORDS;
+        w.sync = (uint32_t *)(w.acc + ACC_WORDS);
+        w.weights = base;
+        std::vector<uint8_t> host(WEIGHT_BYTES);
+        build_weights(host.data());
+        cudaError_t e = slab_wait_polls_address(&w.polls);
+        if (e == cudaSuccess) e = set_attributes();
+        if (e == cudaSuccess) e = make_prod_map(w);
+        if (e == cudaSuccess) e = cudaMemcpy(base, host.data(), host.size(), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) {
+            cudaFree(base);
+            return fail(LUTHE_E_CUDA, "blind rotation setup: %s", cudaGetErrorString(e));
+        }
+        c->ws = w;
+        c->used += bytes;
+    }
+    CUDA_TRY(launch_expand(d_std, c->ws, c->p.lwe_dim, 0));
+    return LUTHE_OK;
 }
 
 int tuning_autoload(luthe_ctx *c);
@@ -129,6 +198,7 @@ extern "C" void luthe_ctx_destroy(luthe_ctx *c)
     if (!c) return;
     cudaSetDevice(c->device);
     drop_graphs(c);
+    brx_release(c);
     const size_t n = c->p.lwe_dim;
     dfree(c, c->d_tw, 4096 * 8);
     dfree(c, c->d_err, 4);
@@ -161,10 +231,11 @@ extern "C" int luthe_upload_bsk(luthe_ctx *c, const uint64_t *h)
     if ((r = dalloc(c, (void **)&d_std, words * 8))) return r;
     cudaError_t e = cudaMemcpy(d_std, h, words * 8, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = launch_bsk_prepare(d_std, c->d_bsk, c->d_tw, (uint32_t)n, 0);
+    if (e == cudaSuccess) r = brx_prepare(c, d_std);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     dfree(c, d_std, words * 8);
     if (e != cudaSuccess) return fail(LUTHE_E_CUDA, "BSK upload: %s", cudaGetErrorString(e));
-    return LUTHE_OK;
+    return r;
 }
 
 extern "C" int luthe_upload_bsk_eval(luthe_ctx *c, const uint64_t *h)
@@ -190,7 +261,20 @@ extern "C" int luthe_upload_bsk_eval(luthe_ctx *c, const uint64_t *h)
     int r;
     if (!c->d_bsk && (r = dalloc(c, (void **)&c->d_bsk, n * SLAB_BYTES))) return r;
     CUDA_TRY(cudaMemcpy(c->d_bsk, slab.data(), words * 8, cudaMemcpyHostToDevice));
-    return LUTHE_OK;
+    // the expanded key is made from the standard domain; it must not outlive the key it was made from
+    uint64_t *d_std = nullptr;
+    const size_t need = words * 8 + (c->ws.weights ? 0 : brx_bytes(c));
+    if (c->used + need > c->budget || dalloc(c, (void **)&d_std, words * 8)) {
+        brx_release(c);
+        return LUTHE_OK;
+    }
+    cudaError_t e = cudaMemcpy(d_std, h, words * 8, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = launch_ntt_inv(d_std, d_std, c->d_tw, n * 4, 0);
+    if (e == cudaSuccess) r = brx_prepare(c, d_std);
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    dfree(c, d_std, words * 8);
+    if (e != cudaSuccess) return fail(LUTHE_E_CUDA, "BSK upload: %s", cudaGetErrorString(e));
+    return r;
 }
 
 extern "C" int luthe_set_tie_rule(luthe_ctx *c, int rule)
@@ -279,14 +363,50 @@ int need_keys(luthe_ctx *c)
     return LUTHE_OK;
 }
 
+// Blind rotation of a whole batch on stream s.  Batches above one ciphertext
+// per SM run on the tensor cores (brx.cu), at most brx::WAVE to a launch: its
+// product tiles want 128 ciphertexts, and a launch of 149 to 296 takes 15 ms
+// against 20 ms of the butterfly kernels' wave (592: 24 ms against 40), one of
+// 100 takes 13 ms against 10.4 ms of the one-per-SM form (148 SMs, n = 804).
+// Smaller batches and remainders run the butterfly kernels.  main_done /
+// main_count as in launch_blind_rotate: the outputs before the last launch.
+static cudaError_t enqueue_blind_rotate(luthe_ctx *c, const uint32_t *d_l2n, const uint32_t *d_ids, uint64_t *d_out,
+                                        size_t count, uint32_t mlk, cudaStream_t s, cudaEvent_t main_done = nullptr,
+                                        size_t *main_count = nullptr)
+{
+    const uint32_t n = c->p.lwe_dim;
+    if (!c->ws.bsk || count <= (size_t)c->nsm)
+        return launch_blind_rotate(c->br, c->nsm, d_l2n, c->d_luts, d_ids, c->nlut, c->d_bsk, c->d_tw, d_out, count, n,
+                                   c->d_err, s, nullptr, mlk, c->p.pbs_base_log, c->tie_rule, main_done, main_count);
+    if (main_count) *main_count = count;
+    for (size_t done = 0; done < count;) {
+        const size_t left = count - done, take = std::min(left, brx::WAVE);
+        if (done && main_done && take == left) {
+            cudaError_t e = cudaEventRecord(main_done, s);
+            if (e != cudaSuccess) return e;
+            if (main_count) *main_count = done;
+        }
+        const uint32_t *l2n = d_l2n + done * (n + 1), *ids = d_ids + done;
+        uint64_t *out = d_out + done * mlk * (size_t)(N + 1);
+        cudaError_t e =
+            take <= (size_t)c->nsm
+                ? launch_blind_rotate(c->br, c->nsm, l2n, c->d_luts, ids, c->nlut, c->d_bsk, c->d_tw, out, take, n,
+                                      c->d_err, s, nullptr, mlk, c->p.pbs_base_log, c->tie_rule)
+                : brx::launch(c->ws, c->nsm, l2n, c->d_luts, ids, c->nlut, out, take, n, c->d_err, s, mlk,
+                              c->p.pbs_base_log, c->tie_rule);
+        if (e != cudaSuccess) return e;
+        done += take;
+    }
+    return cudaSuccess;
+}
+
 static int enqueue_ks_pbs(luthe_ctx *c, const uint64_t *d_in, const uint32_t *d_ids, uint64_t *d_out, size_t count,
                           cudaStream_t s)
 {
     const uint32_t n = c->p.lwe_dim;
     CUDA_TRY(launch_keyswitch(d_in, c->d_ksk, nullptr, c->d_lwe2N, count, n, c->xpad, s, nullptr, c->p.ks_base_log,
                               c->p.ks_level, c->tie_rule, c->d_ks_part));
-    CUDA_TRY(launch_blind_rotate(c->br, c->nsm, c->d_lwe2N, c->d_luts, d_ids, c->nlut, c->d_bsk, c->d_tw, d_out,
-                                 count, n, c->d_err, s, nullptr, 1, c->p.pbs_base_log, c->tie_rule));
+    CUDA_TRY(enqueue_blind_rotate(c, c->d_lwe2N, d_ids, d_out, count, 1, s));
     return LUTHE_OK;
 }
 
@@ -316,8 +436,7 @@ extern "C" int luthe_ks_pbs_ml(luthe_ctx *c, const uint64_t *d_in, const uint32_
     const uint32_t n = c->p.lwe_dim;
     CUDA_TRY(launch_keyswitch(d_in, c->d_ksk, nullptr, c->d_lwe2N, count, n, c->xpad, s, nullptr, c->p.ks_base_log,
                               c->p.ks_level, c->tie_rule, c->d_ks_part));
-    CUDA_TRY(launch_blind_rotate(c->br, c->nsm, c->d_lwe2N, c->d_luts, d_ids, c->nlut, c->d_bsk, c->d_tw, d_out, count,
-                                 n, c->d_err, s, nullptr, mlk, c->p.pbs_base_log, c->tie_rule));
+    CUDA_TRY(enqueue_blind_rotate(c, c->d_lwe2N, d_ids, d_out, count, mlk, s));
     return LUTHE_OK;
 }
 
@@ -382,9 +501,7 @@ static int enqueue_host_ks_pbs(luthe_ctx *c, const uint64_t *h_in, const uint32_
                                   c->d_ks_part));
     }
     size_t full = count;
-    CUDA_TRY(launch_blind_rotate(c->br, c->nsm, c->d_lwe2N, c->d_luts, c->d_hids, c->nlut, c->d_bsk, c->d_tw,
-                                 c->d_hout, count, n, c->d_err, s, nullptr, 1, c->p.pbs_base_log, c->tie_rule,
-                                 c->ev_main, &full));
+    CUDA_TRY(enqueue_blind_rotate(c, c->d_lwe2N, c->d_hids, c->d_hout, count, 1, s, c->ev_main, &full));
     size_t early = 0;  // outputs read back on the copy stream while the tail launch runs
     if (full < count) {
         // the full waves' outputs are final before the tail launch: their
@@ -460,8 +577,7 @@ extern "C" int luthe_blind_rotate(luthe_ctx *c, const uint32_t *d_lwe2N, const u
     if (count == 0) return LUTHE_OK;
     if (!d_lwe2N || !d_ids || !d_out) return fail(LUTHE_E_PARAM, "null buffer");
     CUDA_TRY(cudaSetDevice(c->device));
-    CUDA_TRY(launch_blind_rotate(c->br, c->nsm, d_lwe2N, c->d_luts, d_ids, c->nlut, c->d_bsk, c->d_tw, d_out, count,
-                                 c->p.lwe_dim, c->d_err, (cudaStream_t)stream, nullptr, 1, c->p.pbs_base_log, c->tie_rule));
+    CUDA_TRY(enqueue_blind_rotate(c, d_lwe2N, d_ids, d_out, count, 1, (cudaStream_t)stream));
     return LUTHE_OK;
 }
 
@@ -823,7 +939,6 @@ extern "C" int luthe_ks_pbs_noalloc(luthe_ctx *c, const uint64_t *d_in, const ui
     cudaStream_t s = (cudaStream_t)stream;
     const uint32_t n = c->p.lwe_dim;
     CUDA_TRY(launch_keyswitch(d_in, c->d_ksk, nullptr, scratch, count, n, c->xpad, s, nullptr, c->p.ks_base_log, c->p.ks_level, c->tie_rule));
-    CUDA_TRY(launch_blind_rotate(c->br, c->nsm, scratch, c->d_luts, d_ids, c->nlut, c->d_bsk, c->d_tw, d_out, count, n,
-                                 c->d_err, s, nullptr, 1, c->p.pbs_base_log, c->tie_rule));
+    CUDA_TRY(enqueue_blind_rotate(c, scratch, d_ids, d_out, count, 1, s));
     return LUTHE_OK;
 }

@@ -4,6 +4,7 @@
 #include <stdint.h>
 #include <vector>
 #include "../../include/luthe.h"
+#include "brx.cuh"
 #include "kernels.cuh"
 
 struct GraphEntry {
@@ -39,6 +40,7 @@ struct luthe_ctx {
     cudaEvent_t ev_in = nullptr;         // host path: a chunk of inputs has landed
     luthe::BrConfig br{2, 1};
     uint32_t tie_rule = luthe::TIE_RTL;  // decomposition tie rule (luthe_set_tie_rule)
+    luthe::brx::Workspace ws;            // tensor-core blind rotation; ws.bsk null: not available
     std::vector<GraphEntry> graphs;
 };
 

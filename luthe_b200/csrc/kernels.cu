@@ -477,6 +477,11 @@ cudaError_t set_slab_wait_polls(unsigned long long polls)
     return cudaMemcpyToSymbol(g_slab_wait_polls, &polls, sizeof polls);
 }
 
+cudaError_t slab_wait_polls_address(const unsigned long long **addr)
+{
+    return cudaGetSymbolAddress((void **)addr, g_slab_wait_polls);
+}
+
 __device__ __forceinline__ u32 smem_addr(const void *p) { return (u32)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(u64 *mbar, u32 count)
