@@ -57,19 +57,22 @@ static int check_params(const luthe_params *p)
 }
 
 static void brx_release(luthe_ctx *c);
+static void kstc_release(luthe_ctx *c);
 
 int dalloc(luthe_ctx *c, void **ptr, size_t bytes)
 {
-    // the tensor-core blind rotation's key and workspace are optional: they
-    // give way to anything else the context is asked to hold
+    // the tensor-core forms' keys and buffers are optional: they give way to
+    // anything else the context is asked to hold
     if (c->used + bytes > c->budget) brx_release(c);
+    if (c->used + bytes > c->budget) kstc_release(c);
     if (c->used + bytes > c->budget)
         return fail(LUTHE_E_BUDGET, "HBM budget exceeded: %llu + %zu > %llu bytes", (unsigned long long)c->used,
                     bytes, (unsigned long long)c->budget);
     cudaError_t e = cudaMalloc(ptr, bytes);
-    if (e == cudaErrorMemoryAllocation && c->ws.bsk) {
+    if (e == cudaErrorMemoryAllocation && (c->ws.bsk || c->kt.ksk)) {
         cudaGetLastError();
         brx_release(c);
+        kstc_release(c);
         e = cudaMalloc(ptr, bytes);
     }
     CUDA_TRY(e);
@@ -148,6 +151,65 @@ static int brx_prepare(luthe_ctx *c, const uint64_t *d_std)
     return LUTHE_OK;
 }
 
+// ---- tensor-core key switch: its form of the key and its buffers (ks_tc.cu)
+
+static void kstc_release(luthe_ctx *c)
+{
+    if (!c->kt.ksk) return;
+    drop_graphs(c);
+    cudaFree(c->kt.ksk);  // one allocation
+    c->kt = KsTc{};
+    c->used -= c->kt_bytes;
+    c->kt_bytes = 0;
+}
+
+// Allocate (first key) and fill the key's form from the host KSK.  Without
+// room every key switch runs the dp4a form.  The digit buffer holds 14 row
+// tiles of 256 (140 product CTAs at ten column tiles, one wave), less where
+// the budget is short.
+static int kstc_prepare(luthe_ctx *c, const uint32_t *h)
+{
+    const uint32_t n = c->p.lwe_dim, L = c->p.ks_level;
+    const size_t raw = (size_t)(n + 1) * N * L * 4;
+    const bool fresh = !c->kt.ksk;
+    if (fresh) {
+        const size_t ksk = kstc_ksk_bytes(n, L), part = KSTC_PART_ROWS * (size_t)c->xpad * 4;
+        size_t rows = 3584;
+        while (rows >= 256 && c->used + ksk + part + kstc_digit_bytes(rows, L) + raw > c->budget) rows /= 2;
+        if (rows < 256) return LUTHE_OK;
+        const size_t bytes = ksk + part + kstc_digit_bytes(rows, L);
+        uint8_t *base = nullptr;
+        if (cudaMalloc((void **)&base, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return LUTHE_OK;
+        }
+        c->kt = KsTc{base, base + ksk + part, (uint32_t *)(base + ksk), rows};
+        c->kt_bytes = bytes;
+        c->used += bytes;
+        cudaError_t e = cudaMemset(c->kt.part, 0, part);
+        if (e == cudaSuccess) e = kstc_set_attributes();
+        if (e != cudaSuccess) {
+            kstc_release(c);
+            return fail(LUTHE_E_CUDA, "key switch setup: %s", cudaGetErrorString(e));
+        }
+    }
+    uint32_t *d_raw = nullptr;
+    if (c->used + raw > c->budget || cudaMalloc((void **)&d_raw, raw) != cudaSuccess) {
+        cudaGetLastError();
+        kstc_release(c);  // it must not outlive the key it was made from
+        return LUTHE_OK;
+    }
+    cudaError_t e = cudaMemcpy(d_raw, h, raw, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = launch_kstc_layout(d_raw, c->kt.ksk, n, L, 0);
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    cudaFree(d_raw);
+    if (e != cudaSuccess) {
+        kstc_release(c);
+        return fail(LUTHE_E_CUDA, "KSK upload: %s", cudaGetErrorString(e));
+    }
+    return LUTHE_OK;
+}
+
 int tuning_autoload(luthe_ctx *c);
 
 extern "C" int luthe_ctx_create(const luthe_params *p, int device, uint64_t budget, luthe_ctx **out)
@@ -199,6 +261,7 @@ extern "C" void luthe_ctx_destroy(luthe_ctx *c)
     cudaSetDevice(c->device);
     drop_graphs(c);
     brx_release(c);
+    kstc_release(c);
     const size_t n = c->p.lwe_dim;
     dfree(c, c->d_tw, 4096 * 8);
     dfree(c, c->d_err, 4);
@@ -316,7 +379,7 @@ extern "C" int luthe_upload_ksk(luthe_ctx *c, const uint32_t *h)
         CUDA_TRY(cudaMemset(c->d_ks_part, 0, (size_t)KS_BM * xpad * 4));
     }
     CUDA_TRY(cudaMemcpy(c->d_ksk, t.data(), words * 4, cudaMemcpyHostToDevice));
-    return LUTHE_OK;
+    return kstc_prepare(c, h);
 }
 
 extern "C" int luthe_upload_luts(luthe_ctx *c, const uint64_t *h, uint32_t count)
@@ -400,12 +463,24 @@ static cudaError_t enqueue_blind_rotate(luthe_ctx *c, const uint32_t *d_l2n, con
     return cudaSuccess;
 }
 
+// Key switch of a batch on stream s: on the tensor cores at every size (one
+// BLWE 29 us against 56 us of the split-K dp4a form, 65 of the 2x7 set 31 us
+// against 1.27 ms, 16384 of the 3x6 set: ks_tc.cu), in the dp4a form where the
+// context has no room for the tensor-core form's key.
+static cudaError_t enqueue_keyswitch(luthe_ctx *c, const uint64_t *d_in, uint32_t *d_out21, uint32_t *d_out2N,
+                                     size_t count, cudaStream_t s, uint32_t *d_part)
+{
+    if (c->kt.ksk)
+        return launch_keyswitch_tc(c->kt, c->nsm, d_in, d_out21, d_out2N, count, c->p.lwe_dim, c->xpad, c->p.ks_base_log,
+                                   c->p.ks_level, c->tie_rule, c->d_err, s);
+    return launch_keyswitch(d_in, c->d_ksk, d_out21, d_out2N, count, c->p.lwe_dim, c->xpad, s, nullptr, c->p.ks_base_log,
+                            c->p.ks_level, c->tie_rule, d_part);
+}
+
 static int enqueue_ks_pbs(luthe_ctx *c, const uint64_t *d_in, const uint32_t *d_ids, uint64_t *d_out, size_t count,
                           cudaStream_t s)
 {
-    const uint32_t n = c->p.lwe_dim;
-    CUDA_TRY(launch_keyswitch(d_in, c->d_ksk, nullptr, c->d_lwe2N, count, n, c->xpad, s, nullptr, c->p.ks_base_log,
-                              c->p.ks_level, c->tie_rule, c->d_ks_part));
+    CUDA_TRY(enqueue_keyswitch(c, d_in, nullptr, c->d_lwe2N, count, s, c->d_ks_part));
     CUDA_TRY(enqueue_blind_rotate(c, c->d_lwe2N, d_ids, d_out, count, 1, s));
     return LUTHE_OK;
 }
@@ -433,9 +508,7 @@ extern "C" int luthe_ks_pbs_ml(luthe_ctx *c, const uint64_t *d_in, const uint32_
     CUDA_TRY(cudaSetDevice(c->device));
     if ((r = ensure_scratch(c, count))) return r;
     cudaStream_t s = (cudaStream_t)stream;
-    const uint32_t n = c->p.lwe_dim;
-    CUDA_TRY(launch_keyswitch(d_in, c->d_ksk, nullptr, c->d_lwe2N, count, n, c->xpad, s, nullptr, c->p.ks_base_log,
-                              c->p.ks_level, c->tie_rule, c->d_ks_part));
+    CUDA_TRY(enqueue_keyswitch(c, d_in, nullptr, c->d_lwe2N, count, s, c->d_ks_part));
     CUDA_TRY(enqueue_blind_rotate(c, c->d_lwe2N, d_ids, d_out, count, mlk, s));
     return LUTHE_OK;
 }
@@ -496,9 +569,7 @@ static int enqueue_host_ks_pbs(luthe_ctx *c, const uint64_t *h_in, const uint32_
                                  c->copy_stream));
         CUDA_TRY(cudaEventRecord(c->ev_in, c->copy_stream));
         CUDA_TRY(cudaStreamWaitEvent(s, c->ev_in, 0));
-        CUDA_TRY(launch_keyswitch(c->d_hin + off * row, c->d_ksk, nullptr, c->d_lwe2N + off * (size_t)(n + 1), m,
-                                  n, c->xpad, s, nullptr, c->p.ks_base_log, c->p.ks_level, c->tie_rule,
-                                  c->d_ks_part));
+        CUDA_TRY(enqueue_keyswitch(c, c->d_hin + off * row, nullptr, c->d_lwe2N + off * (size_t)(n + 1), m, s, c->d_ks_part));
     }
     size_t full = count;
     CUDA_TRY(enqueue_blind_rotate(c, c->d_lwe2N, c->d_hids, c->d_hout, count, 1, s, c->ev_main, &full));
@@ -563,9 +634,7 @@ extern "C" int luthe_keyswitch(luthe_ctx *c, const uint64_t *d_in, uint32_t *d_o
     if (count == 0) return LUTHE_OK;
     if (!d_in || !d_out2N) return fail(LUTHE_E_PARAM, "null buffer");
     CUDA_TRY(cudaSetDevice(c->device));
-    CUDA_TRY(launch_keyswitch(d_in, c->d_ksk, d_out21, d_out2N, count, c->p.lwe_dim, c->xpad,
-                              (cudaStream_t)stream, nullptr, c->p.ks_base_log, c->p.ks_level, c->tie_rule,
-                              c->d_ks_part));
+    CUDA_TRY(enqueue_keyswitch(c, d_in, d_out21, d_out2N, count, (cudaStream_t)stream, c->d_ks_part));
     return LUTHE_OK;
 }
 
@@ -937,8 +1006,7 @@ extern "C" int luthe_ks_pbs_noalloc(luthe_ctx *c, const uint64_t *d_in, const ui
         g_noalloc_addr[c->device].store(scratch, std::memory_order_release);
     }
     cudaStream_t s = (cudaStream_t)stream;
-    const uint32_t n = c->p.lwe_dim;
-    CUDA_TRY(launch_keyswitch(d_in, c->d_ksk, nullptr, scratch, count, n, c->xpad, s, nullptr, c->p.ks_base_log, c->p.ks_level, c->tie_rule));
+    CUDA_TRY(enqueue_keyswitch(c, d_in, nullptr, scratch, count, s, nullptr));
     CUDA_TRY(enqueue_blind_rotate(c, scratch, d_ids, d_out, count, 1, s));
     return LUTHE_OK;
 }

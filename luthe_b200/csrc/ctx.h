@@ -41,6 +41,8 @@ struct luthe_ctx {
     luthe::BrConfig br{2, 1};
     uint32_t tie_rule = luthe::TIE_RTL;  // decomposition tie rule (luthe_set_tie_rule)
     luthe::brx::Workspace ws;            // tensor-core blind rotation; ws.bsk null: not available
+    luthe::KsTc kt;                      // tensor-core key switch; kt.ksk null: not available
+    size_t kt_bytes = 0;
     std::vector<GraphEntry> graphs;
 };
 

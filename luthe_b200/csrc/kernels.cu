@@ -3,6 +3,7 @@
 #include <cooperative_groups.h>
 
 #include "kernels.cuh"
+#include "ks_digits.cuh"
 #include "ntt.cuh"
 
 namespace luthe {
@@ -243,32 +244,6 @@ cudaError_t launch_ntt_mul(const uint64_t *d_a, const uint64_t *d_b, uint64_t *d
 // three instructions replace four 32-bit multiply-adds, with two
 // accumulators per output.  Templated
 // on the decomposition (base 2^BL, L levels) of the reference's parameter sets.
-// GEN = false: the RTL's tie rule; GEN = true: the rule of the reference's
-// test-vector generator (TFHE-rs), which takes the digit above the top one as
-// 0, so that a top digit equal to B/2 stays positive.  Both give the same
-// value mod 2^(BL*L); they differ only in that top digit.
-template <int BL, int L, bool GEN>
-__device__ __forceinline__ void ks_decomp(u64 v, int *d)
-{
-    // closest_rep = top BL*L bits + round bit; tie rule of
-    // balanced_decomp_unfix_sign_round_bit.py:42-101 / decomp_parallel.sv:73-75,142-150
-    constexpr int TOT = BL * L;
-    constexpr u32 MASK = (1u << BL) - 1, HALF = 1u << (BL - 1);
-    u32 rb = (u32)(v >> (63 - TOT)) & 1u;
-    u32 c = (u32)(v >> (64 - TOT)) + rb;  // 0 .. 2^TOT
-    u32 last_sign = GEN ? 0u : (((c >> (TOT - 1)) & 1u) && ((c & ((1u << (TOT - 1)) - 1)) || rb));
-    u32 carry = 0;
-#pragma unroll
-    for (int i = 0; i < L; i++) {
-        u32 raw = (c >> (BL * i)) & MASK;
-        u32 nxt = (i + 1 < L) ? ((c >> (BL * (i + 1))) & MASK) : (last_sign ? MASK : 0u);
-        u32 tv = raw + carry;
-        bool negd = (tv >> BL) || ((tv & HALF) && ((tv & (HALF - 1)) || (nxt & HALF)));
-        d[i] = negd ? (int)tv - (1 << BL) : (int)tv;
-        carry = negd ? 1u : 0u;
-    }
-}
-
 // acc + sum over the 4 bytes of (unsigned byte of k) * (signed byte of d)
 __device__ __forceinline__ int dp4a_us(u32 k, u32 d, int acc)
 {
@@ -434,6 +409,14 @@ static cudaError_t launch_keyswitch_rule(const uint64_t *d_in, const uint32_t *d
         const u32 total = B * (n + 1);
         ks_finish<<<(total + 255) / 256, 256, 0, s>>>(d_in, d_src_idx, d_part, d_out21, d_out2N, B, n, xpad);
     }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_ks_finish(const uint64_t *d_in, uint32_t *d_part, uint32_t *d_out21, uint32_t *d_out2N, uint32_t B,
+                             uint32_t n, uint32_t xpad, cudaStream_t s)
+{
+    const u32 total = B * (n + 1);
+    ks_finish<<<(total + 255) / 256, 256, 0, s>>>(d_in, nullptr, d_part, d_out21, d_out2N, B, n, xpad);
     return cudaGetLastError();
 }
 

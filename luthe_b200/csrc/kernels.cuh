@@ -50,6 +50,30 @@ cudaError_t launch_keyswitch(const uint64_t *d_in, const uint32_t *d_ksk_t, uint
 // d_part: KS_BM x xpad u32, all zero, for the split-K form of batches of at
 // most KS_BM ciphertexts (left zero again); nullptr: the one-pass form only.
 // Calls that overlap on the GPU must not share it.
+// The split-K forms' epilogue: outputs of the partial sums, which are cleared.
+cudaError_t launch_ks_finish(const uint64_t *d_in, uint32_t *d_part, uint32_t *d_out21, uint32_t *d_out2N, uint32_t B,
+                             uint32_t n, uint32_t xpad, cudaStream_t s);
+
+// Tensor-core key switch (ks_tc.cu): its form of the KSK and its buffers.
+namespace kstc {
+constexpr int XT = 85;  // outputs of one column tile
+}
+constexpr size_t KSTC_PART_ROWS = 1024;  // largest batch that may split K
+struct KsTc {
+    uint8_t *ksk = nullptr;    // null: not available
+    uint8_t *dig = nullptr;    // digits of `rows` ciphertexts
+    uint32_t *part = nullptr;  // [KSTC_PART_ROWS][xpad] partial sums (kept zero)
+    size_t rows = 0;           // ciphertexts of one pass
+};
+size_t kstc_ksk_bytes(uint32_t n, uint32_t L);
+size_t kstc_digit_bytes(size_t rows, uint32_t L);
+// KSK in the upload's order, on the device -> the tensor-core form
+cudaError_t launch_kstc_layout(const uint32_t *d_ksk, uint8_t *d_dst, uint32_t n, uint32_t L, cudaStream_t s);
+cudaError_t kstc_set_attributes();
+// Calls that overlap on the GPU must not share t's buffers.
+cudaError_t launch_keyswitch_tc(const KsTc &t, int num_sms, const uint64_t *d_in, uint32_t *d_out21, uint32_t *d_out2N,
+                                size_t B, uint32_t n, uint32_t xpad, uint32_t bl, uint32_t L, uint32_t tie_rule,
+                                uint32_t *d_err, cudaStream_t s);
 bool ks_supported(uint32_t bl, uint32_t L);
 bool pbs_supported(uint32_t bw);
 // Bound on the polls of each BSK-slab wait of the blind rotation on the
