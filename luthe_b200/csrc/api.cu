@@ -163,19 +163,17 @@ static void kstc_release(luthe_ctx *c)
     c->kt_bytes = 0;
 }
 
-// Allocate (first key) and fill the key's form from the host KSK.  Without
-// room every key switch runs the dp4a form.  The digit buffer holds 14 row
-// tiles of 256 (140 product CTAs at ten column tiles, one wave), less where
-// the budget is short.
-static int kstc_prepare(luthe_ctx *c, const uint32_t *h)
+// Allocate (first key) and fill the key's form from the KSK as uploaded (d_raw,
+// on the device).  Without room every key switch runs the dp4a form.  The digit
+// buffer holds 14 row tiles of 256 (140 product CTAs at ten column tiles, one
+// wave), less where the budget is short.
+static int kstc_prepare(luthe_ctx *c, const uint32_t *d_raw)
 {
     const uint32_t n = c->p.lwe_dim, L = c->p.ks_level;
-    const size_t raw = (size_t)(n + 1) * N * L * 4;
-    const bool fresh = !c->kt.ksk;
-    if (fresh) {
+    if (!c->kt.ksk) {
         const size_t ksk = kstc_ksk_bytes(n, L), part = KSTC_PART_ROWS * (size_t)c->xpad * 4;
         size_t rows = 3584;
-        while (rows >= 256 && c->used + ksk + part + kstc_digit_bytes(rows, L) + raw > c->budget) rows /= 2;
+        while (rows >= 256 && c->used + ksk + part + kstc_digit_bytes(rows, L) > c->budget) rows /= 2;
         if (rows < 256) return LUTHE_OK;
         const size_t bytes = ksk + part + kstc_digit_bytes(rows, L);
         uint8_t *base = nullptr;
@@ -186,27 +184,10 @@ static int kstc_prepare(luthe_ctx *c, const uint32_t *h)
         c->kt = KsTc{base, base + ksk + part, (uint32_t *)(base + ksk), rows};
         c->kt_bytes = bytes;
         c->used += bytes;
-        cudaError_t e = cudaMemset(c->kt.part, 0, part);
-        if (e == cudaSuccess) e = kstc_set_attributes();
-        if (e != cudaSuccess) {
-            kstc_release(c);
-            return fail(LUTHE_E_CUDA, "key switch setup: %s", cudaGetErrorString(e));
-        }
+        CUDA_TRY(cudaMemset(c->kt.part, 0, part));
+        CUDA_TRY(kstc_set_attributes());
     }
-    uint32_t *d_raw = nullptr;
-    if (c->used + raw > c->budget || cudaMalloc((void **)&d_raw, raw) != cudaSuccess) {
-        cudaGetLastError();
-        kstc_release(c);  // it must not outlive the key it was made from
-        return LUTHE_OK;
-    }
-    cudaError_t e = cudaMemcpy(d_raw, h, raw, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = launch_kstc_layout(d_raw, c->kt.ksk, n, L, 0);
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    cudaFree(d_raw);
-    if (e != cudaSuccess) {
-        kstc_release(c);
-        return fail(LUTHE_E_CUDA, "KSK upload: %s", cudaGetErrorString(e));
-    }
+    CUDA_TRY(launch_kstc_layout(d_raw, c->kt.ksk, n, L, 0));
     return LUTHE_OK;
 }
 
@@ -356,21 +337,10 @@ extern "C" int luthe_upload_ksk(luthe_ctx *c, const uint32_t *h)
 {
     if (!c || !h) return fail(LUTHE_E_PARAM, "null argument");
     CUDA_TRY(cudaSetDevice(c->device));
-    const size_t n = c->p.lwe_dim, K = (size_t)N * c->p.ks_level;
-    const uint32_t xpad = (uint32_t)(((n + 1) + KS_BN - 1) / KS_BN * KS_BN);
-    // device layout [K/4][3][xpad] for the group g = k/4 of four rows: word 0
-    // the low bytes of rows 4g..4g+3, words 1 and 2 their upper 13 bits as
-    // 16-bit halves (rows 4g, 4g+1 and 4g+2, 4g+3)
+    const uint32_t n = c->p.lwe_dim, L = c->p.ks_level;
+    const size_t K = (size_t)N * L, raw = (n + 1) * K * 4;
+    const uint32_t xpad = ((n + 1) + KS_BN - 1) / KS_BN * KS_BN;
     const size_t words = K / 4 * KS_PLANES * xpad;
-    std::vector<uint32_t> t(words, 0);
-    const uint32_t M = (1u << KS_W) - 1;
-    for (size_t x = 0; x <= n; x++)
-        for (size_t k = 0; k < K; k++) {
-            const uint32_t v = h[x * K + k] & M, r = (uint32_t)(k % 4);
-            const size_t g = (k / 4) * KS_PLANES;
-            t[g * xpad + x] |= (v & 0xFFu) << (8 * r);
-            t[(g + 1 + r / 2) * xpad + x] |= (v >> 8) << (16 * (r % 2));
-        }
     int r;
     if (!c->d_ksk) {
         if ((r = dalloc(c, (void **)&c->d_ksk, words * 4))) return r;
@@ -378,8 +348,37 @@ extern "C" int luthe_upload_ksk(luthe_ctx *c, const uint32_t *h)
         if ((r = dalloc(c, (void **)&c->d_ks_part, (size_t)KS_BM * xpad * 4))) return r;
         CUDA_TRY(cudaMemset(c->d_ks_part, 0, (size_t)KS_BM * xpad * 4));
     }
+    // both device forms are made on the device from the key as it came; without
+    // room for that copy the dp4a form is made on the host, and a tensor-core
+    // form of an earlier key must not outlive it
+    uint32_t *d_raw = nullptr;
+    if (c->used + raw <= c->budget && cudaMalloc((void **)&d_raw, raw) == cudaSuccess) {
+        c->used += raw;
+        cudaError_t e = cudaMemcpy(d_raw, h, raw, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = launch_ks_layout(d_raw, c->d_ksk, n, L, xpad, 0);
+        r = e == cudaSuccess ? kstc_prepare(c, d_raw) : LUTHE_OK;
+        const cudaError_t done = cudaDeviceSynchronize();
+        if (e == cudaSuccess) e = done;
+        dfree(c, d_raw, raw);
+        if (e != cudaSuccess || r) kstc_release(c);
+        return e != cudaSuccess ? fail(LUTHE_E_CUDA, "KSK upload: %s", cudaGetErrorString(e)) : r;
+    }
+    cudaGetLastError();
+    kstc_release(c);
+    // device layout [K/4][3][xpad] for the group g = k/4 of four rows: word 0
+    // the low bytes of rows 4g..4g+3, words 1 and 2 their upper 13 bits as
+    // 16-bit halves (rows 4g, 4g+1 and 4g+2, 4g+3)
+    std::vector<uint32_t> t(words, 0);
+    const uint32_t M = (1u << KS_W) - 1;
+    for (size_t x = 0; x <= n; x++)
+        for (size_t k = 0; k < K; k++) {
+            const uint32_t v = h[x * K + k] & M, r4 = (uint32_t)(k % 4);
+            const size_t g = (k / 4) * KS_PLANES;
+            t[g * xpad + x] |= (v & 0xFFu) << (8 * r4);
+            t[(g + 1 + r4 / 2) * xpad + x] |= (v >> 8) << (16 * (r4 % 2));
+        }
     CUDA_TRY(cudaMemcpy(c->d_ksk, t.data(), words * 4, cudaMemcpyHostToDevice));
-    return kstc_prepare(c, h);
+    return LUTHE_OK;
 }
 
 extern "C" int luthe_upload_luts(luthe_ctx *c, const uint64_t *h, uint32_t count)

@@ -67,7 +67,9 @@ struct KsTc {
 };
 size_t kstc_ksk_bytes(uint32_t n, uint32_t L);
 size_t kstc_digit_bytes(size_t rows, uint32_t L);
-// KSK in the upload's order, on the device -> the tensor-core form
+// KSK in the upload's order, on the device -> the dp4a form ([K/4][3][xpad],
+// zero beyond n), the tensor-core form
+cudaError_t launch_ks_layout(const uint32_t *d_ksk, uint32_t *d_dst, uint32_t n, uint32_t L, uint32_t xpad, cudaStream_t s);
 cudaError_t launch_kstc_layout(const uint32_t *d_ksk, uint8_t *d_dst, uint32_t n, uint32_t L, cudaStream_t s);
 cudaError_t kstc_set_attributes();
 // Calls that overlap on the GPU must not share t's buffers.

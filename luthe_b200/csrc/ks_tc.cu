@@ -96,6 +96,25 @@ __global__ void __launch_bounds__(256) layout_kernel(const u32 *__restrict__ ksk
     for (int b = 0; b < 3; b++) o[b] = make_uint4(w[b][0], w[b][1], w[b][2], w[b][3]);
 }
 
+// KSK [x][k] -> the dp4a form, [group of four rows k][3][xpad]: word 0 the low
+// bytes of the rows, words 1 and 2 their upper 13 bits as 16-bit halves
+__global__ void __launch_bounds__(256) dp4a_layout_kernel(const u32 *__restrict__ ksk, u32 *__restrict__ dst, u32 n, u32 groups,
+                                                          u32 xpad)
+{
+    const u32 x = blockIdx.x * 128 + (threadIdx.x & 127), g = blockIdx.y * 2 + (threadIdx.x >> 7);
+    if (g >= groups) return;
+    u32 w[3] = {0, 0, 0};
+    if (x <= n) {
+        const uint4 v = reinterpret_cast<const uint4 *>(ksk)[(size_t)x * groups + g];
+        const u32 M = (1u << KS_W) - 1, r[4] = {v.x & M, v.y & M, v.z & M, v.w & M};
+        w[0] = (r[0] & 0xFF) | (r[1] & 0xFF) << 8 | (r[2] & 0xFF) << 16 | r[3] << 24;
+        w[1] = r[0] >> 8 | r[1] >> 8 << 16;
+        w[2] = r[2] >> 8 | r[3] >> 8 << 16;
+    }
+#pragma unroll
+    for (int p = 0; p < 3; p++) dst[((size_t)g * 3 + p) * xpad + x] = w[p];
+}
+
 // grid: (column tiles, pairs of row tiles, K slices)
 __global__ void __launch_bounds__(THREADS, 1)
     product_kernel(const u64 *__restrict__ in, const uint8_t *__restrict__ dig, const uint8_t *__restrict__ ksk, u32 L,
@@ -238,6 +257,13 @@ cudaError_t launch_kstc_layout(const uint32_t *d_ksk, uint8_t *d_dst, uint32_t n
     if (e != cudaSuccess) return e;
     const u32 total = (n + 1) * (N / 16 * L);
     kstc::layout_kernel<<<(total + 255) / 256, 256, 0, s>>>(d_ksk, d_dst, n, L);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_ks_layout(const uint32_t *d_ksk, uint32_t *d_dst, uint32_t n, uint32_t L, uint32_t xpad, cudaStream_t s)
+{
+    const u32 groups = N * L / 4;
+    kstc::dp4a_layout_kernel<<<dim3(xpad / 128, (groups + 1) / 2), 256, 0, s>>>(d_ksk, d_dst, n, groups, xpad);
     return cudaGetLastError();
 }
 
