@@ -427,9 +427,10 @@ int need_keys(luthe_ctx *c)
 
 // Blind rotation of a whole batch on stream s.  Batches above one ciphertext
 // per SM run on the tensor cores (brx.cu), at most brx::WAVE to a launch: its
-// product tiles want 128 ciphertexts, and a launch of 149 to 296 takes 15 ms
-// against 20 ms of the butterfly kernels' wave (592: 24 ms against 40), one of
-// 100 takes 13 ms against 10.4 ms of the one-per-SM form (148 SMs, n = 804).
+// product tiles want 128 ciphertexts, and a launch of 149 to 296 takes 12.9 to
+// 13.8 ms against 20 ms of the butterfly kernels' wave (592: 21.0 ms against
+// 40), one of 100 takes 12.7 ms against 10.4 ms of the one-per-SM form (148
+// SMs, n = 804).
 // Smaller batches and remainders run the butterfly kernels.  main_done /
 // main_count as in launch_blind_rotate: the outputs before the last launch.
 static cudaError_t enqueue_blind_rotate(luthe_ctx *c, const uint32_t *d_l2n, const uint32_t *d_ids, uint64_t *d_out,

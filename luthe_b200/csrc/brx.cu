@@ -181,12 +181,11 @@ cudaError_t launch_expand(const uint64_t *d_std_p, const Workspace &ws, uint32_t
 // ------------------------------------------------------------------- kernel
 //
 // Sixteen worker warps do all the integer work; one warp each issues the
-// product MMAs and the transform MMAs and copies the product operands; the
-// last one copies products to the inverse transform and publishes finished
+// product MMAs and the transform MMAs, makes the copies, and publishes finished
 // work.  (Twenty warps: five to a scheduler, 96 registers a thread.)
 
 constexpr int WARPS = 16, WORKERS = 32 * WARPS;
-constexpr int W_PMMA = WARPS, W_CMMA = WARPS + 1, W_ATOM = WARPS + 2, W_PROD = WARPS + 3;
+constexpr int W_PMMA = WARPS, W_CMMA = WARPS + 1, W_COPY = WARPS + 2;  // and one that publishes
 constexpr int THREADS = 32 * (WARPS + 4);
 constexpr int STAGES = 5;                  // ring of product operand atoms
 constexpr u32 ATOM = TILE * 128;           // 128 ciphertexts x 128 bytes (16 coefficients)
@@ -194,16 +193,19 @@ constexpr u32 SM_WF = 0, SM_WI = WF_BYTES;
 constexpr u32 SM_BUF = SM_WI + WI_BYTES;
 // first phase: the inverse transform's two operands, then two accumulators; the forward transform's two operands
 constexpr u32 SM_OP = SM_BUF, SM_FOP = SM_BUF + 65536;
-// second phase: the ring; Toeplitz blocks of two units
-constexpr u32 SM_RING = SM_BUF, SM_W = SM_RING + STAGES * ATOM, WSLOT = 16384;
+// second phase: Toeplitz blocks of two units, then the ring; the blocks and the
+// ring's first stages lie where the accumulators were, which are free before
+// the forward transform is done
+constexpr u32 SM_W = SM_BUF, WSLOT = 16384, SM_RING = SM_W + 2 * WSLOT;
+constexpr int EARLY = (65536 - 2 * WSLOT) / ATOM;  // such stages
 constexpr u32 SM_CTL = SM_BUF + 65536 + 49152;
 constexpr u32 SMEM_BYTES = SM_CTL + 256;
-static_assert(SM_RING % 1024 == 0 && SM_W + 2 * WSLOT <= SM_CTL && 2 * BLOCK_BYTES <= WSLOT && SMEM_BYTES <= 232448,
+static_assert(SM_RING % 1024 == 0 && SM_RING + STAGES * ATOM <= SM_CTL && 2 * BLOCK_BYTES <= WSLOT && SMEM_BYTES <= 232448,
               "layout");
 
 // bound on waits that only depend on this CTA's own MMAs and on the drain of
 // copies in flight
-constexpr unsigned long long OWN_POLLS = 1ull << 26;
+constexpr u32 OWN_POLLS = 1u << 26;
 
 struct Ctl {
     u64 full[STAGES], empty[STAGES], wfull[2], wempty[2], dfull[2], dempty[2], opfull, dfree, fop, own[2], drain[2];
@@ -222,32 +224,34 @@ __device__ __forceinline__ void give_up(Ctl *ctl, u32 *sync)
     *(volatile u32 *)&ctl->failed = 1;
     atomicExch(sync, 1u);
 }
-// Bounded waits: by the device-wide number of polls and by about two seconds.
-// They return false once the CTA has given up, so that after a wait ran out
-// anywhere every role runs to its end without blocking.
-constexpr long long WAIT_CLOCKS = 4000000000ll;
+// Bounded waits: by the device-wide number of polls and by about two seconds
+// (counted in 2^10 clocks).  They return false once the CTA has given up, so
+// that after a wait ran out anywhere every role runs to its end without
+// blocking.
+constexpr u32 WAIT_KCLOCKS = 4000000;
 struct Patience {
-    long long t0 = 0;
+    u32 left = WAIT_KCLOCKS, last = (u32)clock();
     // asked every few polls: has this wait lasted too long, or the CTA given up?
     __device__ __forceinline__ bool over(Ctl *ctl)
     {
         if (*(volatile u32 *)&ctl->failed) return true;
-        const long long now = clock64();
-        if (t0 == 0) t0 = now;
-        return now - t0 > WAIT_CLOCKS;
+        const u32 now = (u32)clock(), gone = (now - last) >> 10;
+        last += gone << 10;
+        left -= min(gone, left);
+        return left == 0;
     }
 };
-__device__ __forceinline__ bool wait_bar(u64 *m, u32 parity, unsigned long long polls, Ctl *ctl, u32 *sync)
+__device__ __forceinline__ bool wait_bar(u64 *m, u32 parity, u32 polls, Ctl *ctl, u32 *sync)
 {
-    const u32 a = tc::smem_u32(m);
+    if (polls && tc::mbar_test(m, parity)) return true;
     Patience patience;
-    for (unsigned long long it = 0; it < polls; it++) {
+    for (u32 it = 0; it < polls; it++) {
         u32 done;
         asm volatile("{\n\t.reg .pred p;\n\t"
                      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
                      "selp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(done)
-                     : "r"(a), "r"(parity)
+                     : "r"(tc::smem_u32(m)), "r"(parity)
                      : "memory");
         if (done) return true;
         if ((it & 7) == 7 && patience.over(ctl)) break;
@@ -273,22 +277,12 @@ __device__ __forceinline__ u32 load_relaxed(const u32 *p)
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(got) : "l"(p) : "memory");
     return got;
 }
-__device__ __forceinline__ bool wait_smem(u32 *p, u32 want, unsigned long long polls, Ctl *ctl, u32 *sync)
+__device__ __forceinline__ bool wait_smem(u32 *p, u32 want, u32 polls, Ctl *ctl, u32 *sync)
 {
     Patience patience;
-    for (unsigned long long it = 0; it < polls; it++) {
+    for (u32 it = 0; it < polls; it++) {
         if (smem_count(p) >= want) return true;
         if ((it & 15) == 15 && patience.over(ctl)) break;
-    }
-    give_up(ctl, sync);
-    return false;
-}
-__device__ __forceinline__ bool wait_grid(const u32 *p, u32 want, unsigned long long polls, Ctl *ctl, u32 *sync)
-{
-    Patience patience;
-    for (unsigned long long it = 0; it < polls; it++) {
-        if (load_acquire(p) >= want) return true;
-        if ((it & 15) == 15 && (patience.over(ctl) || load_relaxed(sync))) break;
     }
     give_up(ctl, sync);
     return false;
@@ -410,7 +404,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     Ctl *ctl = reinterpret_cast<Ctl *>(sm + SM_CTL);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const u32 smem = tc::smem_u32(sm);
-    const unsigned long long polls = *polls_p;
+    const u32 polls = (u32)min(*polls_p, 0xFFFFFFFFull);
 
     if (tid == 0) {
         for (int i = 0; i < STAGES; i++) {
@@ -440,15 +434,19 @@ __global__ void __launch_bounds__(THREADS, 1)
     tc::fence_after();
     const u32 tmem = ctl->tmem;  // columns 0-255 and 256-511: points z_m and 1/z_m; units in turn
     const Plan pl = make_plan(B);
-    u32 ring = 0, blocks = 0;  // atoms and units' blocks moved (copy and MMA warps)
+    u32 ring = 0, blocks = 0, gathers = 0;  // atoms, units' blocks and couples' products moved (copy and MMA warps)
 
     if (warp < WARPS) {
         // ------------------------------------------------------------ workers
         const int r = tid & 127, cq = tid >> 7;  // MMA row (TMEM lane); quarter of the columns
-        const int cl = r >> 6, q = (r >> 5) & 1, x = r & 31;  // ciphertext of the pair, polynomial (column), coefficient mod 32
+        // row = polynomial (column), pair of coefficients mod 32, ciphertext of the couple, coefficient of the pair: the
+        // order in which the products' 64-byte pieces (two ciphertexts) land
+        const int q = r >> 6, cl = (r >> 1) & 1, x = ((r & 63) >> 2) * 2 + (r & 1);
         const u32 lane_base = (u32)(r & ~31) << 16;
         const u32 tie_floor = tie_rule == TIE_RTL ? 1u << (31 - BW) : 0u;
-        u64 *accs = reinterpret_cast<u64 *>(sm + SM_OP);  // [2][2][N]: takes the operands' place once they are consumed
+        // [2][2][N]: takes the operands' place once they are consumed; the second ciphertext's words are swapped in
+        // eights (index ^ 8), so that a warp's 16 words of each lie in different banks
+        u64 *accs = reinterpret_cast<u64 *>(sm + SM_OP);
         u64 z[16];  // accumulator at x + 32 j: j = 8 cq + e, then j + 32
         u64 held[8];  // products at the first point of a pair
         u32 own = 0, useq = 0;
@@ -463,28 +461,25 @@ __global__ void __launch_bounds__(THREADS, 1)
             tc::fence_after();
         };
         auto acc_of = [&](u32 pair) { return acc_g + (size_t)(2 * pair + cl) * 2 * N + q * N + x + XN * 8 * cq; };
-        auto fetch_acc = [&](u32 pair) {
-            const u64 *ac = acc_of(pair);
-#pragma unroll
-            for (int e = 0; e < 16; e++) z[e] = __ldcg(ac + XN * ((e & 7) + (e >> 3) * PH));
-        };
-
         // One step of a pair of ciphertexts.
-        auto step_pair = [&](u32 i, u32 pair, u32 next, bool next_loads) {
+        auto step_pair = [&](u32 i, u32 pair) {
             const u32 ct = 2 * pair + cl, ctv = min(ct, B - 1);  // the last pair may be half empty
             u64 *acc = acc_of(pair);
-            u64 *as = accs + (cl * 2 + q) * N + x + XN * 8 * cq;
+            u64 *as = accs + (cl * 2 + q) * N + (x ^ (cl * 8)) + XN * 8 * cq;
             const u32 a = lwe2N[(size_t)ctv * (n + 1) + i];
             if (i == 0) {
                 u32 lid = lut_id[ctv];
                 if (lid >= nlut) {  // device-resident ids cannot be checked by the host: flag it, stay in bounds
-                    if (r % 64 == 0 && cq == 0) atomicOr(err, DEVERR_LUT_ID);
+                    if (q == 0 && x == 0 && cq == 0) atomicOr(err, DEVERR_LUT_ID);
                     lid = 0;
                 }
                 const u64 *lut = luts + (size_t)lid * 2 * N + q * N + x + XN * 8 * cq;
 #pragma unroll
                 for (int e = 0; e < 16; e++) z[e] = lut[XN * ((e & 7) + (e >> 3) * PH)];
             } else {
+                // (loaded here, under the inverse transform; ahead of it they would cost another stage its registers)
+#pragma unroll
+                for (int e = 0; e < 16; e++) z[e] = __ldcg(acc + XN * ((e & 7) + (e >> 3) * PH));
                 // E_j in columns 8 j, G_{31-j} in columns 256 + 8 (31 - j)
                 wait_own(cq >> 1);
                 const u32 src_e = tmem + lane_base + cq * 64, src_g = tmem + lane_base + 256 + (24 - 8 * cq) * 8;
@@ -543,12 +538,12 @@ __global__ void __launch_bounds__(THREADS, 1)
                         for (int e = 0; e < 8; e++) {
                             const u32 oi = t + 256 * e;
                             const u32 src = ((oi == 0 ? 0u : (u32)N - oi) + b) & (TWO_N - 1);
-                            u64 w = ag[src & (N - 1)];
+                            u64 w = ag[(src & (N - 1)) ^ (g * 8)];
                             if (src >= (u32)N) w = 0ull - w;
                             __stcs((unsigned long long *)o + oi, oi == 0 ? w : 0ull - w);
                         }
                         if (t == 0) {
-                            const u64 w = ag[N + (b & (N - 1))];
+                            const u64 w = ag[N + ((b & (N - 1)) ^ (g * 8))];
                             __stcs((unsigned long long *)o + N, b >= (u32)N ? 0ull - w : w);
                         }
                     }
@@ -556,7 +551,6 @@ __global__ void __launch_bounds__(THREADS, 1)
                 tc::fence_async_smem();
                 arrive(&ctl->dfree);
                 if (lane == 0) add_smem(&ctl->freed);
-                if (next_loads) fetch_acc(next);
                 return;
             }
             // rotate, subtract, decompose: the digits of 8 pairs (j, j + 32) of this row, twice 48 bytes: in order
@@ -572,7 +566,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     for (int f = 0; f < 8; f++) {
                         const u32 p = src + ((u32)(XN * (f + g * PH)) << 20);
                         const u64 m = (u64)(int64_t)((int32_t)p >> 31);  // upper half: negated
-                        const u64 rot = ap[(p >> 20) & (N - 1)];
+                        const u64 rot = ap[((p >> 20) & (N - 1)) ^ (cl * 8)];
                         hi[f] = (u32)(((rot ^ m) - z[8 * g + f] - m) >> 32);
                     }
                     digits8<BW>(hi, tie_floor, d + 8 * g);
@@ -593,7 +587,6 @@ __global__ void __launch_bounds__(THREADS, 1)
             tc::fence_async_smem();
             arrive(&ctl->fop);
             if (lane == 0) add_smem(&ctl->freed);  // the rotation has read accs: the next operands may land there
-            if (next_loads) fetch_acc(next);
             // evaluations -> the product's operand: atom (polynomial, 16 coefficients), row = ciphertext,
             // K reversed (slot 31 - x), 128-byte swizzle
             const u32 slot = XN - 1 - x, row = ct & (TILE - 1);
@@ -669,9 +662,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 
         for (u32 i = 0; i <= n; i++) {
             for (u32 m = 0; m < pl.couples; m++) {
-                const bool wrap = m + 1 >= pl.couples;
-                const u32 ni = wrap ? i + 1 : i;
-                step_pair(i, blockIdx.x + m * gridDim.x, blockIdx.x + (wrap ? 0 : m + 1) * gridDim.x, ni > 0 && ni <= n);
+                step_pair(i, blockIdx.x + m * gridDim.x);
             }
             for (u32 m = 0; m < pl.units && i < n; m++) drain(get_unit(pl, m));
         }
@@ -685,7 +676,9 @@ __global__ void __launch_bounds__(THREADS, 1)
             for (u32 i = 0; i < n && good; i++)
                 for (u32 m = 0; m < pl.units && good; m++) {
                     const u32 d = blocks & 1, dt = tmem + d * 256;
-                    if (blocks >= 2) good = wait_bar(&ctl->dempty[d], ((blocks >> 1) - 1) & 1, polls, ctl, sync);
+                    // the forward transforms' accumulators lie where the units' go
+                    if (m == 0) good = wait_smem(&ctl->cts_done, WARPS * pl.couples * (i + 1), polls, ctl, sync);
+                    if (blocks >= 2) good = good && wait_bar(&ctl->dempty[d], ((blocks >> 1) - 1) & 1, polls, ctl, sync);
                     good = good && wait_bar(&ctl->wfull[d], (blocks >> 1) & 1, polls, ctl, sync);
                     const u64 wd0 = tc::desc_at(dw, d * WSLOT);
 #pragma unroll
@@ -763,14 +756,49 @@ __global__ void __launch_bounds__(THREADS, 1)
                     __syncwarp();
                 }
             }
-    } else if (warp == W_ATOM) {
-        // ------------------------------------------------- product operands, once their tile is complete
+    } else if (warp == W_COPY) {
+        // ------------------------------------------------- copies: a couple's products to the inverse transform
+        // once its tile's units are done, then the units' operands once their tile is complete
         bool good = true;
         const u32 tiles = (B + TILE - 1) / TILE;
-        for (u32 i = 0; i < n && good; i++) {
-            // the ring lies in the first phase's buffers
-            if (pl.units) good = __all_sync(0xFFFFFFFFu, wait_smem(&ctl->cts_done, WARPS * pl.couples * (i + 1), polls, ctl, sync));
-            u32 complete = 0;  // tiles seen complete in this step: each lane watches one
+        u32 seq = 0;  // couples so far
+        // each lane watches one tile's counter; false if that wait ran out
+        auto wait_tile = [&](u32 tile, u32 &complete, bool units, u32 i) {
+            Patience patience;
+            for (u32 it = 0; !(complete >> tile & 1); it++) {
+                const u32 t = min((u32)lane, tiles - 1);
+                const u32 got = load_acquire(units ? unit_count(sync, t) : ct_count(sync, t));
+                complete = __ballot_sync(0xFFFFFFFFu, got >= (units ? PK * 2 * i : tile_cts(B, t) * (i + 1)));
+                const bool over = it >= polls || ((it & 15) == 15 && (patience.over(ctl) || load_relaxed(sync)));
+                if (__any_sync(0xFFFFFFFFu, over) && !(complete >> tile & 1)) {
+                    give_up(ctl, sync);
+                    return false;
+                }
+            }
+            return true;
+        };
+        for (u32 i = 0; i <= n && good; i++) {
+            u32 complete = 0;
+            for (u32 m = 0; m < pl.couples && good; m++, seq++) {
+                if (i == 0) continue;
+                const u32 ct = 2 * (blockIdx.x + m * gridDim.x);
+                // this CTA's units are drained (their operands lay here), the last couple's accumulators read
+                if (m == 0) good = wait_smem(&ctl->units_done, WARPS * pl.units * i, polls, ctl, sync);
+                good = good && wait_smem(&ctl->freed, WARPS * seq, polls, ctl, sync);
+                good = __all_sync(0xFFFFFFFFu, good) && wait_tile(ct / TILE, complete, true, i);
+                if (good && lane == 0) {
+                    tc::fence_async_global();
+                    tc::mbar_expect_tx(&ctl->opfull, 65536);
+                    // each lands as [pair of points][column, pair of x][ciphertext][x][2]
+                    tc::tensor_g2s(sm + SM_OP, &prod_map, (ct & (TILE - 1)) / 2, ct / TILE * PH, &ctl->opfull);
+                    tc::tensor_g2s(sm + SM_OP + 32768, &prod_map, (ct & (TILE - 1)) / 2, ct / TILE * PH + PH / 2, &ctl->opfull);
+                    gathers++;
+                }
+            }
+            if (i == n || !pl.units || !good) continue;
+            good = __all_sync(0xFFFFFFFFu, wait_smem(&ctl->freed, WARPS * seq, polls, ctl, sync));
+            complete = 0;
+            u32 first = 0;  // atoms of this step
             for (u32 m = 0; m < pl.units && good; m++) {
                 const Unit u = get_unit(pl, m);
                 const u32 slot = blocks & 1;
@@ -783,92 +811,42 @@ __global__ void __launch_bounds__(THREADS, 1)
                                  2 * BLOCK_BYTES, &ctl->wfull[slot]);
                 }
                 blocks++;
-                Patience patience;
-                for (unsigned long long it = 0; !(complete >> u.tile & 1); it++) {
-                    const u32 t = min((u32)lane, tiles - 1);
-                    complete = __ballot_sync(0xFFFFFFFFu, load_acquire(ct_count(sync, t)) >= tile_cts(B, t) * (i + 1));
-                    const bool over = it >= polls || ((it & 15) == 15 && (patience.over(ctl) || load_relaxed(sync)));
-                    if (__any_sync(0xFFFFFFFFu, over)) {
-                        give_up(ctl, sync);
-                        good = false;
-                        break;
-                    }
-                }
+                good = wait_tile(u.tile, complete, false, i);
                 if (lane == 0) {
                     tc::fence_async_global();
                     const u64 *src = ev + (size_t)u.tile * TILE_WORDS + (size_t)u.p * 4 * (ATOM / 8);
-                    for (u32 a = 0; a < 4 && good; a++) {
+                    for (u32 a = 0; a < 4 && good; a++, first++) {
                         const u32 st = ring % STAGES;
-                        if (ring >= STAGES) good = wait_bar(&ctl->empty[st], (ring / STAGES - 1) & 1, polls, ctl, sync);
+                        // a stage where the digits lay waits for the forward transforms, as does one of the last step
+                        if (first < (u32)STAGES && st >= (u32)EARLY)
+                            good = wait_smem(&ctl->cts_done, WARPS * seq, polls, ctl, sync);
+                        if (good && ring >= STAGES) good = wait_bar(&ctl->empty[st], (ring / STAGES - 1) & 1, polls, ctl, sync);
                         if (!good) break;
                         tc::mbar_expect_tx(&ctl->full[st], ATOM);
                         tc::bulk_g2s(sm + SM_RING + st * ATOM, src + a * (ATOM / 8), ATOM, &ctl->full[st]);
                         ring++;
                     }
                 }
-                __syncwarp();
+                good = __all_sync(0xFFFFFFFFu, good);
             }
         }
     } else {
-        // Two tasks in one loop that never blocks: publish finished pairs and
-        // units in the workers' order, and copy a pair's products into the
-        // operand buffers once its tile's units are done (and this CTA's,
-        // whose ring lies there).
+        // ------------------------------------------------- publish finished couples and units, in the workers' order
         if (lane == 0) {
-            u32 pi = 1, pm = 0, pseq = pl.couples;        // next copy: step, position, pairs before it
-            u32 cts = 0, units = 0;                     // events published
-            u32 ci = 0, cm = 0, ui = 0, um = 0, part = 0;
-            bool copying = pl.couples > 0, publishing = true;
-            unsigned long long idle = 0;
-            Patience patience;
-            while ((copying || publishing) && !*(volatile u32 *)&ctl->failed) {
-                bool did = false;
-                if (copying) {
-                    const u32 ct = 2 * (blockIdx.x + pm * gridDim.x);
-                    if (smem_count(&ctl->freed) >= WARPS * pseq && smem_count(&ctl->units_done) >= WARPS * pl.units * pi &&
-                        load_acquire(unit_count(sync, ct / TILE)) >= PK * 2 * pi) {
-                        tc::fence_async_global();
-                        tc::mbar_expect_tx(&ctl->opfull, 65536);
-                        // gathers of 32-byte pieces; each lands as [pair of points][ciphertext, column, x][2]
-                        tc::tensor_g2s(sm + SM_OP, &prod_map, ct & (TILE - 1), ct / TILE * PH, &ctl->opfull);
-                        tc::tensor_g2s(sm + SM_OP + 32768, &prod_map, ct & (TILE - 1), ct / TILE * PH + PH / 2, &ctl->opfull);
-                        ring++;
-                        pseq++;
-                        did = true;
-                        if (++pm == pl.couples) pm = 0, copying = ++pi <= n;
-                    }
+            u32 cts = 0, units = 0;
+            bool good = true;
+            for (u32 i = 0; i < n && good; i++) {
+                for (u32 m = 0; m < pl.couples && good; m++) {
+                    const u32 ct = 2 * (blockIdx.x + m * gridDim.x);
+                    good = wait_smem(&ctl->cts_done, WARPS * ++cts, polls, ctl, sync);
+                    if (good) publish(ct_count(sync, ct / TILE), min(2u, B - ct));
                 }
-                if (publishing) {
-                    bool adv = true;
-                    if (part == 0) {
-                        if (cm < pl.couples) {
-                            adv = smem_count(&ctl->cts_done) >= WARPS * (cts + 1);
-                            if (adv) {
-                                const u32 ct = 2 * (blockIdx.x + cm * gridDim.x);
-                                publish(ct_count(sync, ct / TILE), min(2u, B - ct));
-                                cts++;
-                            }
-                        }
-                    } else if (um < pl.units) {
-                        adv = smem_count(&ctl->units_done) >= WARPS * (units + 1);
-                        if (adv) {
-                            const Unit u = get_unit(pl, um);
-                            if (u.alone || (u.p & 1)) publish(unit_count(sync, u.tile), u.alone ? 1 : 2);
-                            units++;
-                        }
-                    }
-                    if (adv) {
-                        did = true;
-                        if (part == 0) {
-                            if (++cm >= pl.couples) cm = 0, ci++, part = 1;
-                        } else {
-                            if (++um >= pl.units) um = 0, ui++, part = 0, publishing = ui < n;
-                        }
-                    }
+                for (u32 m = 0; m < pl.units && good; m++) {
+                    const Unit u = get_unit(pl, m);
+                    good = wait_smem(&ctl->units_done, WARPS * ++units, polls, ctl, sync);
+                    // the products of a pair of points leave with its second unit
+                    if (good && (u.alone || (u.p & 1))) publish(unit_count(sync, u.tile), u.alone ? 1 : 2);
                 }
-                idle = did ? 0 : idle + 1;
-                if (did) patience.t0 = 0;
-                else if (idle >= polls || ((idle & 15) == 15 && (patience.over(ctl) || load_relaxed(sync)))) give_up(ctl, sync);
             }
         }
     }
@@ -884,13 +862,12 @@ __global__ void __launch_bounds__(THREADS, 1)
             const int k = warp - W_PMMA;
             tc::commit(&ctl->drain[k]);
             drained = tc::mbar_wait(&ctl->drain[k], 0, OWN_POLLS);
-        } else if (tid == W_ATOM * 32) {
+        } else if (tid == W_COPY * 32) {
             for (u32 s = 0; s < STAGES; s++)
                 if (ring > s) drained &= tc::mbar_wait(&ctl->full[s], ((ring - 1 - s) / STAGES) & 1, OWN_POLLS);
             for (u32 s = 0; s < 2; s++)
                 if (blocks > s) drained &= tc::mbar_wait(&ctl->wfull[s], ((blocks - 1 - s) >> 1) & 1, OWN_POLLS);
-        } else if (tid == W_PROD * 32) {
-            if (ring) drained = tc::mbar_wait(&ctl->opfull, (ring - 1) & 1, OWN_POLLS);
+            if (gathers) drained &= tc::mbar_wait(&ctl->opfull, (gathers - 1) & 1, OWN_POLLS);
         }
         if (tid == 0) atomicOr(err, DEVERR_TIMEOUT);
         if (!drained) atomicOr(err, DEVERR_DRAIN);
@@ -910,9 +887,10 @@ cudaError_t set_attributes()
     return e;
 }
 
-// The products as a tensor of 32-byte pieces: (8 words, pair of outputs,
-// ciphertext of the tile, (tile, pair of points)); a box is the pieces of two
-// ciphertexts at 16 pairs of points.
+// The products as a tensor of 64-byte pieces (a pair of outputs at a pair of
+// points, of two ciphertexts): (16 words, pair of outputs, couple of the tile,
+// (tile, pair of points)); a box is a couple's pieces at 16 pairs of points.
+// (One ciphertext's 32-byte pieces took 5,000 clocks for the 64 KB.)
 static_assert(sizeof(TensorMap) == sizeof(CUtensorMap) && alignof(TensorMap) >= alignof(CUtensorMap), "tensor map");
 cudaError_t make_prod_map(Workspace &ws)
 {
@@ -921,9 +899,9 @@ cudaError_t make_prod_map(Workspace &ws)
     cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found);
     if (e != cudaSuccess) return e;
     if (found != cudaDriverEntryPointSuccess || !fn) return cudaErrorNotSupported;
-    const cuuint64_t dims[4] = {8, (cuuint64_t)XN, (cuuint64_t)TILE, TILES * PH};
-    const cuuint64_t strides[3] = {32 * TILE, 32, 32 * TILE * XN};  // bytes, of dimensions 1 to 3
-    const cuuint32_t box[4] = {8, (cuuint32_t)XN, 2, PH / 2}, step[4] = {1, 1, 1, 1};
+    const cuuint64_t dims[4] = {16, (cuuint64_t)XN, (cuuint64_t)TILE / 2, TILES * PH};
+    const cuuint64_t strides[3] = {32 * TILE, 64, 32 * TILE * XN};  // bytes, of dimensions 1 to 3
+    const cuuint32_t box[4] = {16, (cuuint32_t)XN, 1, PH / 2}, step[4] = {1, 1, 1, 1};
     const CUresult r = reinterpret_cast<decltype(&cuTensorMapEncodeTiled)>(fn)(
         reinterpret_cast<CUtensorMap *>(&ws.prod_map), CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, ws.prod, dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
