@@ -219,6 +219,7 @@ extern "C" int luthe_ctx_create(const luthe_params *p, int device, uint64_t budg
     if (e == cudaSuccess) e = cudaMemset(c->d_err, 0, 4);
     if (e == cudaSuccess) e = br_set_attributes(BrConfig{1, 1}, p->lwe_dim);
     if (e == cudaSuccess) e = br_set_attributes(BrConfig{2, 1}, p->lwe_dim);
+    if (e == cudaSuccess) e = br_cluster_limits(&c->br);
     if (e == cudaSuccess) {
         // diagnostics: LUTHE_SLAB_WAIT_POLLS bounds each BSK-slab wait (0: run out at once)
         const char *polls = getenv("LUTHE_SLAB_WAIT_POLLS");
@@ -691,6 +692,8 @@ extern "C" int luthe_set_br_config(luthe_ctx *c, int g, int per_sm)
     if (!c) return fail(LUTHE_E_PARAM, "null ctx");
     if (g < 1 || g > 2 || per_sm < 1) return fail(LUTHE_E_PARAM, "bad BR config %d/%d", g, per_sm);
     BrConfig cfg{g, per_sm};
+    cfg.oct_max = c->br.oct_max;
+    cfg.quad_max = c->br.quad_max;
     CUDA_TRY(cudaSetDevice(c->device));
     size_t smem = br_smem_bytes(cfg, c->p.lwe_dim);
     int max_smem = 0;
@@ -729,7 +732,8 @@ extern "C" int luthe_check_device_error(luthe_ctx *c)
 // launch_blind_rotate): ciphertexts per CTA (G), and the batch sizes up to
 // which a batch runs one ciphertext per 2-SM cluster (pair_max) or one per
 // CTA (split_max), and up to which a partial last wave runs as its own launch
-// of those forms (tail_max).  The autotuner times every form around each
+// of those forms (tail_max).  (The larger clusters of the smallest batches are
+// bounded by what fits at once, not tuned.)  The autotuner times every form around each
 // decision point on this device and keeps the fastest; the choice can be
 // saved as JSON and loaded by later contexts (the counterpart of the HPU's
 // batch configuration, pep_sequencer.sv:573-620 and docs/hpu_parameters.md).

@@ -300,26 +300,6 @@ __device__ __forceinline__ void publish(u32 *p, u32 count)
 }
 __device__ __forceinline__ void workers_bar() { asm volatile("bar.sync 1, %0;" ::"n"(WORKERS) : "memory"); }
 
-// v + the p -> 2^64 switch of a lazy residue a (gl::modsw_p_to_q of its
-// canonical form): a + a_hi + [a_lo > 2^31 + [a >= 2^63]].  A lazy a = p + e,
-// e < 2^32 - 1, has a_hi = 2^32 - 1 and a_lo = e + 1, and the same sum gives
-// e + [e > 2^31] mod 2^64, the switch of e.
-__device__ __forceinline__ u64 add_modsw(u64 v, u64 a)
-{
-    const u64 s = v + a;
-    const u32 hi = (u32)(a >> 32), k = 0x7FFFFFFFu - (hi >> 31);
-    u64 r;
-    asm("{\n\t.reg .u32 x, s0, s1;\n\t"
-        "mov.b64 {s0, s1}, %1;\n\t"
-        "add.cc.u32 x, %2, %3;\n\t"
-        "addc.cc.u32 s0, s0, %4;\n\t"
-        "addc.u32 s1, s1, 0;\n\t"
-        "mov.b64 %0, {s0, s1};\n\t}"
-        : "=l"(r)
-        : "l"(s), "r"((u32)a), "r"(k), "r"(hi));
-    return r;
-}
-
 // Balanced digits of eight 64-bit torus words whose upper halves are hi[], base
 // 2^BW, one level (gl::decomp_to_p), as 24-bit words of three signed bytes.
 // Rounding bit, sign and wrap are one addition: z / 2^(32-BW) is d + 2^(BW-1)
@@ -510,8 +490,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                         s[3] = tc::lift(3) + v[0] + v[2];
                         u64 c0, c1;
                         tc::fold2_lifted(t, s, c0, c1);
-                        z[e + f] = add_modsw(z[e + f], c0);
-                        z[8 + e + f] = add_modsw(z[8 + e + f], c1);
+                        z[e + f] = gl::add_modsw(z[e + f], c0);
+                        z[8 + e + f] = gl::add_modsw(z[8 + e + f], c1);
                     }
                 }
                 tc::fence_before();

@@ -256,6 +256,26 @@ __device__ __forceinline__ u64 modsw_p_to_q(u64 a)
     return a + ((hx + 0x80000000ull) >> 32);
 }
 
+// v + the p -> 2^64 switch of a lazy residue a (modsw_p_to_q of its
+// canonical form): a + a_hi + [a_lo > 2^31 + [a >= 2^63]].  A lazy a = p + e,
+// e < 2^32 - 1, has a_hi = 2^32 - 1 and a_lo = e + 1, and the same sum gives
+// e + [e > 2^31] mod 2^64, the switch of e.
+__device__ __forceinline__ u64 add_modsw(u64 v, u64 a)
+{
+    const u64 s = v + a;
+    const u32 hi = (u32)(a >> 32), k = 0x7FFFFFFFu - (hi >> 31);
+    u64 r;
+    asm("{\n\t.reg .u32 x, s0, s1;\n\t"
+        "mov.b64 {s0, s1}, %1;\n\t"
+        "add.cc.u32 x, %2, %3;\n\t"
+        "addc.cc.u32 s0, s0, %4;\n\t"
+        "addc.u32 s1, s1, 0;\n\t"
+        "mov.b64 %0, {s0, s1};\n\t}"
+        : "=l"(r)
+        : "l"(s), "r"((u32)a), "r"(k), "r"(hi));
+    return r;
+}
+
 // Balanced decomposition, base 2^23, one level, of a 64-bit torus value,
 // embedded in Z_p (decomp_balseq_core.sv:135-150; the rounding and tie rule of
 // sw/decomposer/balanced_decomp_unfix_sign_round_bit.py:42-101 with bw=23, L=1).

@@ -926,8 +926,8 @@ __device__ __forceinline__ void issue_half_slab_warp(u64 *hs, const u64 *src, u3
 // share an SM.
 constexpr size_t PAIR_SMEM_BYTES = 132 * 1024;
 
-// Lowest-latency form, for batches of at most one ciphertext per two SMs: a
-// cluster of two CTAs (256 threads each, one per SM) per ciphertext, CTA r
+// Low-latency form, for batches of at most one ciphertext per two SMs (the
+// smallest run on larger clusters, br_parts.cuh): a cluster of two CTAs (256 threads each, one per SM) per ciphertext, CTA r
 // owning polynomial r -- the split form above with the two groups on two
 // SMs.  Each CTA streams only its half of the slab (column r); for the BSK
 // multiply each CTA stores its forward transform into a receive buffer in the
@@ -1102,6 +1102,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
     cluster.sync();  // no CTA leaves while the other may still address its shared memory
 }
 
+}  // namespace luthe
+#include "br_parts.cuh"
+namespace luthe {
+
 size_t br_smem_bytes(const BrConfig &cfg, uint32_t n)
 {
     const int G = cfg.cts_per_cta;
@@ -1139,16 +1143,26 @@ cudaError_t br_set_attributes(const BrConfig &cfg, uint32_t n)
     }
 }
 
+cudaError_t br_cluster_limits(BrConfig *cfg)
+{
+    cudaError_t e = parts::prepare(4, &cfg->oct_max);
+    return e == cudaSuccess ? parts::prepare(2, &cfg->quad_max) : e;
+}
+
 // One blind-rotation launch.  G: ciphertexts per CTA (1 or 2, br_kernel);
 // 0: one ciphertext per CTA split over its two groups (br_kernel_split);
-// -1: one ciphertext per cluster of two CTAs (br_kernel_pair).
+// -1: one ciphertext per cluster of two CTAs (br_kernel_pair); -2, -4: one
+// ciphertext per cluster of 4 or 8 CTAs (br_parts.cuh).
 static cudaError_t launch_br_once(int G, int ctas_per_sm, int nsm, const uint32_t *d_lwe2N, const uint64_t *d_luts,
                                   const uint32_t *d_lut_id, uint32_t nlut, const uint64_t *d_bsk,
                                   const uint64_t *d_tw, uint64_t *d_out, size_t B, uint32_t n, uint32_t *d_err,
                                   cudaStream_t s, const uint32_t *d_dst_idx, uint32_t mlk, uint32_t pbs_bw,
                                   uint32_t tie_rule)
 {
-    if (G == -1) {  // lowest-latency form: a cluster of two CTAs (two SMs) per ciphertext
+    if (G < -1)
+        return parts::launch(-G, d_lwe2N, d_luts, d_lut_id, nlut, d_bsk, d_tw, d_out, B, n, d_err, s, d_dst_idx, mlk,
+                             pbs_bw, tie_rule);
+    if (G == -1) {  // low-latency form: a cluster of two CTAs (two SMs) per ciphertext
         size_t pairs = B < (size_t)(nsm / 2) ? B : (size_t)(nsm / 2);
         u32 Bu = (u32)B;
         void *args[] = {(void *)&d_lwe2N, (void *)&d_luts, (void *)&d_lut_id, (void *)&nlut, (void *)&d_bsk,
@@ -1204,9 +1218,16 @@ cudaError_t launch_blind_rotate(const BrConfig &cfg, int nsm, const uint32_t *d_
     // A batch that fits one ciphertext per SM runs in the latency form (one
     // ciphertext per CTA, its polynomials split over the two groups): with
     // G = 2 ciphertexts per CTA half the SMs would idle.
-    // At most one ciphertext per two SMs: the two-SM form, lower latency still.
+    // At most one ciphertext per two SMs: the two-SM form, lower latency still,
+    // and clusters of more SMs for the smallest batches.
     // (Both forms are persistent over their ciphertexts, so any cut-off is correct.)
-    auto small_form = [&](size_t count) { return count <= pair_max ? -1 : 0; };
+    // As many as fit at the same time go on clusters of eight or four SMs (15 and
+    // 33 on 148 SMs: 3.0 and 4.3 ms against 6.8 ms of the two-SM form; the 16th
+    // would wait for a whole bootstrap, 6.0 ms).
+    auto small_form = [&](size_t count) {
+        if (count > pair_max) return 0;
+        return count <= (size_t)cfg.oct_max ? -4 : count <= (size_t)cfg.quad_max ? -2 : -1;
+    };
     if (G > 1 && B <= split_max)
         return launch_br_once(small_form(B), 1, nsm, d_lwe2N, d_luts, d_lut_id, nlut, d_bsk, d_tw, d_out, B, n,
                               d_err, s, d_dst_idx, mlk, pbs_bw, tie_rule);

@@ -27,6 +27,9 @@ struct BrConfig {
     int pair_max = -1;   // batches up to this run one ciphertext per 2-SM cluster (default SMs / 2)
     int split_max = -1;  // ... else up to this, one ciphertext per CTA (default SMs)
     int tail_max = -1;   // a partial last wave up to this runs as its own small launch (default SMs)
+    // batches of at most pair_max up to these sizes run one ciphertext per
+    // 8-SM or 4-SM cluster (br_cluster_limits: as many as are resident at once)
+    int oct_max = 0, quad_max = 0;
 };
 
 // device twiddle tables: [fwd 8x256][inv 8x256]
@@ -91,6 +94,7 @@ cudaError_t launch_blind_rotate(const BrConfig &cfg, int num_sms, const uint32_t
                                 size_t *main_count = nullptr);
 size_t br_smem_bytes(const BrConfig &cfg, uint32_t n);
 cudaError_t br_set_attributes(const BrConfig &cfg, uint32_t n);
+cudaError_t br_cluster_limits(BrConfig *cfg);  // sets oct_max and quad_max for the current device
 
 enum LweOp : int { LWE_ADD = 0, LWE_SUB = 1, LWE_MAC = 2, LWE_ADDS = 3, LWE_SUBS = 4, LWE_SSUB = 5, LWE_MULS = 6 };
 // one linear DOp or register copy (op = LWE_COPY) on slots of a BLWE pool

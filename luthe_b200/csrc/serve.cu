@@ -563,15 +563,18 @@ extern "C" int luthe_server_step(luthe_server *s, uint32_t *n_completed, uint32_
             }
             r->ready.swap(keep);
         }
-        // Cluster pairs hold two SMs per ciphertext for about 7 ms.  When the
-        // ciphertexts already on the GPU and this batch would need more SMs
-        // than there are, pairs would queue for SMs; the batch then runs one
-        // ciphertext per CTA instead (10.4 ms on one SM: about 40 % more
-        // bootstraps per SM-second).
+        // Clusters hold eight, four or two SMs per ciphertext for 3.0, 4.3 or
+        // 6.9 ms.  When the ciphertexts already on the GPU and this batch
+        // would need more SMs than there are, clusters would queue for SMs;
+        // the batch then takes the next smaller cluster, in the end one
+        // ciphertext per CTA (10.4 ms on one SM: about 40 % more bootstraps
+        // per SM-second than pairs).
         size_t inflight = 0;
         for (const Lane &o : s->lanes)
             if (o.busy) inflight += o.ops.size();
         BrConfig cfg = c->br;
+        if (8 * (inflight + B) > (size_t)c->nsm) cfg.oct_max = 0;
+        if (4 * (inflight + B) > (size_t)c->nsm) cfg.quad_max = 0;
         if (2 * (inflight + B) > (size_t)c->nsm) cfg.pair_max = 0;
         CUDA_TRY(cudaStreamWaitEvent(ln.stream, s->alu_done, 0));
         CUDA_TRY(cudaMemcpyAsync(ln.d_idx, ln.h_idx, (size_t)s->max_pbs * 3 * 4, cudaMemcpyHostToDevice, ln.stream));
