@@ -37,7 +37,9 @@
  *    pre-transformed from the host: hw/module/bsk/module/bsk_manager), and,
  *    where the HBM budget has room for it, to the operand form of the
  *    tensor-core blind rotation (2.0 MB per LWE coefficient and 63 MB of
- *    workspace; given up again when a later allocation needs the room).
+ *    workspace; given up again when a later allocation needs the room, but for
+ *    forms that launches captured by the caller use: those stay until the
+ *    context ends and no longer count against the budget).
  *  - LUT:  trivial GLWE, mask polynomial then body polynomial, natural order.
  */
 #ifndef LUTHE_H

@@ -56,16 +56,26 @@ static int check_params(const luthe_params *p)
     return LUTHE_OK;
 }
 
+static size_t brx_bytes(const luthe_ctx *c);
 static void brx_release(luthe_ctx *c);
 static void kstc_release(luthe_ctx *c);
+
+// Bytes of the tensor-core forms that launches captured by the caller use: they
+// stay where they are until the context ends, and stop counting against the
+// budget, which would otherwise refuse what they used to give way to.
+static size_t held_bytes(const luthe_ctx *c)
+{
+    return (c->ws_held ? brx_bytes(c) : 0) + (c->kt_held ? c->kt_bytes : 0);
+}
+static bool over_budget(const luthe_ctx *c, size_t bytes) { return c->used - held_bytes(c) + bytes > c->budget; }
 
 int dalloc(luthe_ctx *c, void **ptr, size_t bytes)
 {
     // the tensor-core forms' keys and buffers are optional: they give way to
     // anything else the context is asked to hold
-    if (c->used + bytes > c->budget) brx_release(c);
-    if (c->used + bytes > c->budget) kstc_release(c);
-    if (c->used + bytes > c->budget)
+    if (over_budget(c, bytes)) brx_release(c);
+    if (over_budget(c, bytes)) kstc_release(c);
+    if (over_budget(c, bytes))
         return fail(LUTHE_E_BUDGET, "HBM budget exceeded: %llu + %zu > %llu bytes", (unsigned long long)c->used,
                     bytes, (unsigned long long)c->budget);
     cudaError_t e = cudaMalloc(ptr, bytes);
@@ -104,7 +114,7 @@ static size_t brx_bytes(const luthe_ctx *c)
 
 static void brx_release(luthe_ctx *c)
 {
-    if (!c->ws.weights) return;
+    if (!c->ws.weights || c->ws_held) return;
     drop_graphs(c);  // captured launches use the workspace
     cudaFree(c->ws.weights);  // one allocation
     c->ws = brx::Workspace{};
@@ -121,7 +131,7 @@ static int brx_prepare(luthe_ctx *c, const uint64_t *d_std)
         const size_t bytes = brx_bytes(c);
         int cooperative = 0;
         CUDA_TRY(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, c->device));
-        if (!cooperative || c->used + bytes > c->budget) return LUTHE_OK;
+        if (!cooperative || over_budget(c, bytes)) return LUTHE_OK;
         uint8_t *base = nullptr;
         if (cudaMalloc((void **)&base, bytes) != cudaSuccess) {
             cudaGetLastError();
@@ -155,7 +165,7 @@ static int brx_prepare(luthe_ctx *c, const uint64_t *d_std)
 
 static void kstc_release(luthe_ctx *c)
 {
-    if (!c->kt.ksk) return;
+    if (!c->kt.ksk || c->kt_held) return;
     drop_graphs(c);
     cudaFree(c->kt.ksk);  // one allocation
     c->kt = KsTc{};
@@ -173,7 +183,7 @@ static int kstc_prepare(luthe_ctx *c, const uint32_t *d_raw)
     if (!c->kt.ksk) {
         const size_t ksk = kstc_ksk_bytes(n, L), part = KSTC_PART_ROWS * (size_t)c->xpad * 4;
         size_t rows = 3584;
-        while (rows >= 256 && c->used + ksk + part + kstc_digit_bytes(rows, L) > c->budget) rows /= 2;
+        while (rows >= 256 && over_budget(c, ksk + part + kstc_digit_bytes(rows, L))) rows /= 2;
         if (rows < 256) return LUTHE_OK;
         const size_t bytes = ksk + part + kstc_digit_bytes(rows, L);
         uint8_t *base = nullptr;
@@ -242,6 +252,7 @@ extern "C" void luthe_ctx_destroy(luthe_ctx *c)
     if (!c) return;
     cudaSetDevice(c->device);
     drop_graphs(c);
+    c->ws_held = c->kt_held = false;
     brx_release(c);
     kstc_release(c);
     const size_t n = c->p.lwe_dim;
@@ -309,7 +320,10 @@ extern "C" int luthe_upload_bsk_eval(luthe_ctx *c, const uint64_t *h)
     // the expanded key is made from the standard domain; it must not outlive the key it was made from
     uint64_t *d_std = nullptr;
     const size_t need = words * 8 + (c->ws.weights ? 0 : brx_bytes(c));
-    if (c->used + need > c->budget || dalloc(c, (void **)&d_std, words * 8)) {
+    if (c->ws_held) {  // captured launches read it: it has to follow the key
+        CUDA_TRY(cudaMalloc((void **)&d_std, words * 8));
+        c->used += words * 8;
+    } else if (over_budget(c, need) || dalloc(c, (void **)&d_std, words * 8)) {
         brx_release(c);
         return LUTHE_OK;
     }
@@ -353,7 +367,7 @@ extern "C" int luthe_upload_ksk(luthe_ctx *c, const uint32_t *h)
     // room for that copy the dp4a form is made on the host, and a tensor-core
     // form of an earlier key must not outlive it
     uint32_t *d_raw = nullptr;
-    if (c->used + raw <= c->budget && cudaMalloc((void **)&d_raw, raw) == cudaSuccess) {
+    if ((c->kt_held || !over_budget(c, raw)) && cudaMalloc((void **)&d_raw, raw) == cudaSuccess) {
         c->used += raw;
         cudaError_t e = cudaMemcpy(d_raw, h, raw, cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = launch_ks_layout(d_raw, c->d_ksk, n, L, xpad, 0);
@@ -365,6 +379,7 @@ extern "C" int luthe_upload_ksk(luthe_ctx *c, const uint32_t *h)
         return e != cudaSuccess ? fail(LUTHE_E_CUDA, "KSK upload: %s", cudaGetErrorString(e)) : r;
     }
     cudaGetLastError();
+    if (c->kt_held) return fail(LUTHE_E_CUDA, "KSK upload: no device memory for the key's copy");
     kstc_release(c);
     // device layout [K/4][3][xpad] for the group g = k/4 of four rows: word 0
     // the low bytes of rows 4g..4g+3, words 1 and 2 their upper 13 bits as
@@ -426,6 +441,18 @@ int need_keys(luthe_ctx *c)
     return LUTHE_OK;
 }
 
+// A launch that the caller captures may be replayed whenever they like: what it
+// uses is held.  (The context's own graphs are dropped with what they use.)
+static bool captured(luthe_ctx *c, cudaStream_t s)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+        cudaGetLastError();  // the launch itself reports it
+        return false;
+    }
+    return st == cudaStreamCaptureStatusActive && !c->own_capture;
+}
+
 // Blind rotation of a whole batch on stream s.  Batches above one ciphertext
 // per SM run on the tensor cores (brx.cu), at most brx::WAVE to a launch: its
 // product tiles want 128 ciphertexts, and a launch of 149 to 296 takes 12.9 to
@@ -443,6 +470,7 @@ static cudaError_t enqueue_blind_rotate(luthe_ctx *c, const uint32_t *d_l2n, con
         return launch_blind_rotate(c->br, c->nsm, d_l2n, c->d_luts, d_ids, c->nlut, c->d_bsk, c->d_tw, d_out, count, n,
                                    c->d_err, s, nullptr, mlk, c->p.pbs_base_log, c->tie_rule, main_done, main_count);
     if (main_count) *main_count = count;
+    c->ws_held |= captured(c, s);
     for (size_t done = 0; done < count;) {
         const size_t left = count - done, take = std::min(left, brx::WAVE);
         if (done && main_done && take == left) {
@@ -471,9 +499,11 @@ static cudaError_t enqueue_blind_rotate(luthe_ctx *c, const uint32_t *d_l2n, con
 static cudaError_t enqueue_keyswitch(luthe_ctx *c, const uint64_t *d_in, uint32_t *d_out21, uint32_t *d_out2N,
                                      size_t count, cudaStream_t s, uint32_t *d_part)
 {
-    if (c->kt.ksk)
+    if (c->kt.ksk) {
+        c->kt_held |= captured(c, s);
         return launch_keyswitch_tc(c->kt, c->nsm, d_in, d_out21, d_out2N, count, c->p.lwe_dim, c->xpad, c->p.ks_base_log,
                                    c->p.ks_level, c->tie_rule, c->d_err, s);
+    }
     return launch_keyswitch(d_in, c->d_ksk, d_out21, d_out2N, count, c->p.lwe_dim, c->xpad, s, nullptr, c->p.ks_base_log,
                             c->p.ks_level, c->tie_rule, d_part);
 }
@@ -532,7 +562,9 @@ extern "C" int luthe_ks_pbs_graph(luthe_ctx *c, const uint64_t *d_in, const uint
         }
     cudaGraph_t graph;
     CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    c->own_capture = true;
     r = enqueue_ks_pbs(c, d_in, d_ids, d_out, count, s);
+    c->own_capture = false;
     cudaError_t e = cudaStreamEndCapture(s, &graph);
     if (r) return r;
     if (e != cudaSuccess) return fail(LUTHE_E_CUDA, "graph capture: %s", cudaGetErrorString(e));

@@ -43,6 +43,8 @@ struct luthe_ctx {
     luthe::brx::Workspace ws;            // tensor-core blind rotation; ws.bsk null: not available
     luthe::KsTc kt;                      // tensor-core key switch; kt.ksk null: not available
     size_t kt_bytes = 0;
+    bool ws_held = false, kt_held = false;  // used by launches that the caller captured
+    bool own_capture = false;               // a graph of luthe_ks_pbs_graph is being captured
     std::vector<GraphEntry> graphs;
 };
 
