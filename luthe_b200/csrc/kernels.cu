@@ -82,150 +82,95 @@ cudaError_t launch_bsk_prepare(const uint64_t *d_std_p, uint64_t *d_slab, const 
 
 // ------------------------------------------------------------ standalone NTT
 //
-// G polynomials (or pairs) per CTA, 256 threads each; the twiddle tables are
-// staged once per CTA in shared memory.
-
-template <int G>
-__device__ __forceinline__ void load_tw(u64 *tws, const u64 *__restrict__ tw, int words)
-{
-    for (int i = threadIdx.x; i < words; i += G * TPG) tws[i] = tw[i];
-}
+// One polynomial (or pair) to a CTA of 256 threads.  A thread needs eight words
+// of the twiddle table, the same in every CTA, and reads them from L1 or L2 where
+// the pass uses them; staging the table in shared memory, for two polynomials a
+// CTA, put a copy and a barrier before the first pass (one transform 7.8 us, now
+// 4.9).  The grid is as long as the batch, so that SMs take the next
+// polynomial as they finish one: a persistent grid left the SMs with an uneven
+// number of them (333: 13.9 us, now 10.2; 1000: 25.3, now 20.5).
+// Bound: the integer ALU; 4096 transforms take 74 to 77 us (85 to 87 before), of
+// which 20 us are the transfers at the copy's rate; 4096 products 219 us (233).
 
 // forward: coefficient order in, evaluation order k out (A_k = A(psi^{2k+1}))
-template <int G>
-__global__ void __launch_bounds__(G * 256) ntt_fwd_kernel(const u64 *__restrict__ in, u64 *__restrict__ out,
-                                                           const u64 *__restrict__ tw, size_t count)
+__global__ void __launch_bounds__(TPG, 4) ntt_fwd_kernel(const u64 *__restrict__ in, u64 *__restrict__ out,
+                                                         const u64 *__restrict__ tw)
 {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    u64 *tws = reinterpret_cast<u64 *>(smem_raw);
-    u64 *buf = tws + 2048 + (threadIdx.x >> 8) * POLY_WORDS;
-    load_tw<G>(tws, tw, 2048);
-    __syncthreads();
-    const int t = threadIdx.x & 255, bar = 1 + (threadIdx.x >> 8);
-    for (size_t poly = (size_t)blockIdx.x * G + (threadIdx.x >> 8); poly < ((count + G - 1) / G) * G;
-         poly += (size_t)gridDim.x * G) {
-        const size_t src = poly < count ? poly : count - 1;
-        u64 x[1][8];
+    __shared__ u64 buf[POLY_WORDS];
+    const int t = threadIdx.x;
+    const size_t at = (size_t)blockIdx.x * N;
+    u64 x[1][8];
 #pragma unroll
-        for (int e = 0; e < 8; e++) x[0][e] = in[src * N + ntt::coef_index(t, e)];
-        ntt::forward<1>(x, buf, tws, t, bar);
-        if (poly < count) {
+    for (int e = 0; e < 8; e++) x[0][e] = in[at + ntt::coef_index(t, e)];
+    ntt::forward<1>(x, buf, tw, t, 1);
 #pragma unroll
-            for (int p = 0; p < 8; p++) out[poly * N + ntt::eval_index(t, p)] = gl::canon(x[0][p]);
-        }
-        ntt::group_sync(bar);
-    }
+    for (int p = 0; p < 8; p++) out[at + ntt::eval_index(t, p)] = gl::canon(x[0][p]);
 }
 
 // inverse: evaluation order in, coefficient order out, with the 1/N factor
-template <int G>
-__global__ void __launch_bounds__(G * 256) ntt_inv_kernel(const u64 *__restrict__ in, u64 *__restrict__ out,
-                                                           const u64 *__restrict__ tw, size_t count)
+__global__ void __launch_bounds__(TPG, 4) ntt_inv_kernel(const u64 *__restrict__ in, u64 *__restrict__ out,
+                                                         const u64 *__restrict__ tw)
 {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    u64 *tws = reinterpret_cast<u64 *>(smem_raw);
-    u64 *buf = tws + 2048 + (threadIdx.x >> 8) * POLY_WORDS;
-    load_tw<G>(tws, tw + 2048, 2048);
-    __syncthreads();
-    const int t = threadIdx.x & 255, bar = 1 + (threadIdx.x >> 8);
-    for (size_t poly = (size_t)blockIdx.x * G + (threadIdx.x >> 8); poly < ((count + G - 1) / G) * G;
-         poly += (size_t)gridDim.x * G) {
-        const size_t src = poly < count ? poly : count - 1;
-        u64 x[1][8];
+    __shared__ u64 buf[POLY_WORDS];
+    const int t = threadIdx.x;
+    const size_t at = (size_t)blockIdx.x * N;
+    u64 x[1][8];
 #pragma unroll
-        for (int p = 0; p < 8; p++) x[0][p] = gl::div2k(in[src * N + ntt::eval_index(t, p)], 11);  // x N^-1 = x 2^-11
-        ntt::inverse<1>(x, buf, tws, t, bar);
-        if (poly < count) {
+    for (int p = 0; p < 8; p++) x[0][p] = gl::div2k(in[at + ntt::eval_index(t, p)], 11);  // x N^-1 = x 2^-11
+    ntt::inverse<1>(x, buf, tw + 2048, t, 1);
 #pragma unroll
-            for (int e = 0; e < 8; e++) out[poly * N + ntt::coef_index(t, e)] = gl::canon(x[0][e]);
-        }
-        ntt::group_sync(bar);
-    }
+    for (int e = 0; e < 8; e++) out[at + ntt::coef_index(t, e)] = gl::canon(x[0][e]);
 }
 
 // negacyclic product of pairs: INTT(NTT(a) * NTT(b))
-template <int G>
-__global__ void __launch_bounds__(G * 256, 2) ntt_mul_kernel(const u64 *__restrict__ a, const u64 *__restrict__ b,
-                                                           u64 *__restrict__ out, const u64 *__restrict__ tw,
-                                                           size_t count)
+__global__ void __launch_bounds__(TPG, 4) ntt_mul_kernel(const u64 *__restrict__ a, const u64 *__restrict__ b,
+                                                         u64 *__restrict__ out, const u64 *__restrict__ tw)
 {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    u64 *tws = reinterpret_cast<u64 *>(smem_raw);
-    u64 *buf = tws + 4096 + (threadIdx.x >> 8) * 2 * POLY_WORDS;
-    load_tw<G>(tws, tw, 4096);
-    __syncthreads();
-    const int t = threadIdx.x & 255, bar = 1 + (threadIdx.x >> 8);
-    for (size_t pr = (size_t)blockIdx.x * G + (threadIdx.x >> 8); pr < ((count + G - 1) / G) * G;
-         pr += (size_t)gridDim.x * G) {
-        const size_t src = pr < count ? pr : count - 1;
-        u64 x[2][8];
+    __shared__ u64 buf[2 * POLY_WORDS];
+    const int t = threadIdx.x;
+    const size_t at = (size_t)blockIdx.x * N;
+    u64 x[2][8];
 #pragma unroll
-        for (int e = 0; e < 8; e++) {
-            x[0][e] = a[src * N + ntt::coef_index(t, e)];
-            x[1][e] = b[src * N + ntt::coef_index(t, e)];
-        }
-        ntt::forward<2>(x, buf, tws, t, bar);
-        u64 r[1][8];
-#pragma unroll
-        for (int p = 0; p < 8; p++) r[0][p] = gl::div2k(gl::mul(x[0][p], x[1][p]), 11);  // N^-1 = 2^-11: one exact division
-        ntt::group_sync(bar);
-        ntt::inverse<1>(r, buf, tws + 2048, t, bar);
-        if (pr < count) {
-#pragma unroll
-            for (int e = 0; e < 8; e++) out[pr * N + ntt::coef_index(t, e)] = gl::canon(r[0][e]);
-        }
-        ntt::group_sync(bar);
+    for (int e = 0; e < 8; e++) {
+        x[0][e] = a[at + ntt::coef_index(t, e)];
+        x[1][e] = b[at + ntt::coef_index(t, e)];
     }
+    ntt::forward<2>(x, buf, tw, t, 1);
+    u64 r[1][8];
+#pragma unroll
+    for (int p = 0; p < 8; p++) r[0][p] = gl::div2k(gl::mul(x[0][p], x[1][p]), 11);  // N^-1 = 2^-11: one exact division
+    ntt::group_sync(1);
+    ntt::inverse<1>(r, buf, tw + 2048, t, 1);
+#pragma unroll
+    for (int e = 0; e < 8; e++) out[at + ntt::coef_index(t, e)] = gl::canon(r[0][e]);
 }
 
-static int num_sms()
-{
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
-}
-
-template <typename K>
-static cudaError_t launch_grid(K kernel, int G, size_t smem, size_t units, const void *const *args,
-                               cudaStream_t s)
-{
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, G * TPG, smem);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    size_t want = (units + G - 1) / G;
-    size_t grid = (size_t)per_sm * num_sms();
-    if (grid > want) grid = want;
-    if (grid == 0) grid = 1;
-    return cudaLaunchKernel((const void *)kernel, dim3((unsigned)grid), dim3(G * TPG), (void **)args, smem, s);
-}
+// launches of at most as many CTAs as a grid may have
+constexpr size_t MAX_GRID = 0x7FFFFFFF;
 
 cudaError_t launch_ntt_fwd(const uint64_t *d_in, uint64_t *d_out, const uint64_t *d_tw, size_t count,
                            cudaStream_t s)
 {
     if (count == 0) return cudaSuccess;
-    constexpr int G = 2;
-    const void *args[] = {&d_in, &d_out, &d_tw, &count};
-    return launch_grid(ntt_fwd_kernel<G>, G, (2048 + G * POLY_WORDS) * 8, count, args, s);
+    if (count > MAX_GRID) return cudaErrorInvalidValue;
+    ntt_fwd_kernel<<<(unsigned)count, TPG, 0, s>>>(d_in, d_out, d_tw);
+    return cudaGetLastError();
 }
 cudaError_t launch_ntt_inv(const uint64_t *d_in, uint64_t *d_out, const uint64_t *d_tw, size_t count,
                            cudaStream_t s)
 {
     if (count == 0) return cudaSuccess;
-    constexpr int G = 2;
-    const void *args[] = {&d_in, &d_out, &d_tw, &count};
-    return launch_grid(ntt_inv_kernel<G>, G, (2048 + G * POLY_WORDS) * 8, count, args, s);
+    if (count > MAX_GRID) return cudaErrorInvalidValue;
+    ntt_inv_kernel<<<(unsigned)count, TPG, 0, s>>>(d_in, d_out, d_tw);
+    return cudaGetLastError();
 }
 cudaError_t launch_ntt_mul(const uint64_t *d_a, const uint64_t *d_b, uint64_t *d_out, const uint64_t *d_tw,
                            size_t count, cudaStream_t s)
 {
     if (count == 0) return cudaSuccess;
-    constexpr int G = 2;
-    const void *args[] = {&d_a, &d_b, &d_out, &d_tw, &count};
-    return launch_grid(ntt_mul_kernel<G>, G, (4096 + G * 2 * POLY_WORDS) * 8, count, args, s);
+    if (count > MAX_GRID) return cudaErrorInvalidValue;
+    ntt_mul_kernel<<<(unsigned)count, TPG, 0, s>>>(d_a, d_b, d_out, d_tw);
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------- key switch
