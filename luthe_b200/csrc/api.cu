@@ -493,8 +493,8 @@ static cudaError_t enqueue_blind_rotate(luthe_ctx *c, const uint32_t *d_l2n, con
 }
 
 // Key switch of a batch on stream s: on the tensor cores at every size (one
-// BLWE 29 us against 56 us of the split-K dp4a form, 65 of the 2x7 set 31 us
-// against 1.27 ms, 16384 of the 3x6 set: ks_tc.cu), in the dp4a form where the
+// BLWE 23 us against 56 us of the split-K dp4a form, 65 of the 2x7 set 27 us
+// against 1.27 ms, 16384 of the 3x6 set 0.54 ms against 10.35: ks_tc.cu), in the dp4a form where the
 // context has no room for the tensor-core form's key.
 static cudaError_t enqueue_keyswitch(luthe_ctx *c, const uint64_t *d_in, uint32_t *d_out21, uint32_t *d_out2N,
                                      size_t count, cudaStream_t s, uint32_t *d_part)

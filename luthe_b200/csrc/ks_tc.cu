@@ -1,4 +1,4 @@
-// Key switch on the tensor cores, for batches above the split-K form's 32.
+// Key switch on the tensor cores.
 //
 //   out21[c][x] = [x == n] b21 - sum_{y,z} d_{c,y,z} KSK[y][z][x]  (mod 2^21)
 //
@@ -8,8 +8,7 @@
 // tcgen05 kind::i8, M = ciphertexts, N = (x, byte), K = (coefficient, level).
 //
 // The digits are made once, by a kernel of their own, in the operand's layout:
-// the product has ten column tiles, and each would make them again (about 50
-// instructions per coefficient, more than the MMAs' own time).  A product CTA
+// the product has ten column tiles, and each would make them again.  A product CTA
 // takes 256 ciphertexts x 85 outputs (255 of 256 columns; both accumulators
 // fill TMEM): per 32 K bytes it moves 16 KB for 256 clocks of MMA, a square
 // tile being the one that needs least from L2, which at 41 bytes per clock and
@@ -17,15 +16,14 @@
 // and add their partial sums into a buffer (32-bit wrap-around sums are exact
 // mod 2^21 in any order).
 //
-// One B200, n = 804, KS 3x6: 16384 BLWEs in 0.60 ms against 10.35 ms with
-// dp4a/dp2a on the multiply pipe (per pass of 3584: digits 37 us, product 91 us,
+// One B200, n = 804, KS 3x6: 16384 BLWEs in 0.54 ms against 10.35 ms with
+// dp4a/dp2a on the multiply pipe (per pass of 3584: digits 26 us, product 91 us,
 // 450 clocks per K step where L2 would allow 390 and the MMAs 256), 65 BLWEs of
-// the 2x7 set 31 us against 1.27 ms.
+// the 2x7 set 27 us against 1.27 ms.
 #include <algorithm>
 
 #include "kernels.cuh"
 #include "tc.cuh"
-#include "ks_digits.cuh"
 
 namespace luthe {
 namespace kstc {
@@ -51,41 +49,121 @@ struct Ctl {
 };
 static_assert(sizeof(Ctl) <= 256, "control block");
 
-// digits of 128 ciphertexts x 32 coefficients: [level][half][row][16 coefficients]
+// Order of the coefficients along K: a warp's word of digits holds coefficients
+// l, l + 32, l + 64, l + 96 of a run of 128 (lane l), so that it reads whole rows
+// and packs four digits without an exchange; a K block is eight such words.
+__device__ __forceinline__ u32 k_coef(u32 blk, u32 slot)
+{
+    return (blk >> 2) * 128 + (blk & 3) * 8 + (slot >> 2) + (slot & 3) * 32;
+}
+
+template <int BL>
+__host__ __device__ constexpr u32 fields(u32 v, int count)  // v in each of the lowest fields of BL bits
+{
+    u32 p = 0;
+    for (int i = 0; i < count; i++) p |= v << (BL * i);
+    return p;
+}
+// All balanced digits of a torus word (its upper half) at once, as ks_decomp
+// (ks_digits.cuh): digit z is field z of s, less HALF - 1, less field z of e.
+// e is the rule of a tie, raw digit + carry = B/2: negative where the raw digit
+// above has its top bit; for the top digit (RTL's rule) where its own top bit is
+// set and the word is not exactly the tie without a rounding bit.  Adding
+// HALF - 1 + e to every field makes the carries those of the decomposition.
+template <int BL, int L, bool GEN>
+__device__ __forceinline__ void digit_fields(u32 hi, u32 &s, u32 &e)
+{
+    constexpr int TOT = BL * L;
+    const u32 t = hi >> (31 - TOT), c = (t + 1) >> 1;
+    e = (c >> (2 * BL - 1)) & fields<BL>(1, L - 1);
+    if (!GEN && t != (1u << TOT)) e |= (c >> (BL - 1)) & (1u << (BL * (L - 1)));
+    s = c + fields<BL>((1u << (BL - 1)) - 1, L) + e;
+}
+// byte k of w[j] = byte j of v[k], j < 3
+__device__ __forceinline__ void transpose(const u32 (&v)[4], u32 (&w)[3])
+{
+    const u32 a = __byte_perm(v[0], v[1], 0x5140), b = __byte_perm(v[2], v[3], 0x5140);
+    w[0] = __byte_perm(a, b, 0x5410);
+    w[1] = __byte_perm(a, b, 0x7632);
+    w[2] = __byte_perm(__byte_perm(v[0], v[1], 0x0062), __byte_perm(v[2], v[3], 0x0062), 0x5410);
+}
+// BITS bits from bit AT of four words whose bytes were transposed, a byte each
+template <int AT, int BITS>
+__device__ __forceinline__ u32 field4(const u32 (&w)[3])
+{
+    constexpr u32 ONES = 0x01010101u;
+    constexpr int J = AT / 8, O = AT % 8;
+    if constexpr (O + BITS <= 8) {
+        return (w[J] >> O) & (((1u << BITS) - 1) * ONES);
+    } else {
+        constexpr int LO = 8 - O;
+        return ((w[J] >> O) & (((1u << LO) - 1) * ONES)) | ((w[J + 1] & (((1u << (BITS - LO)) - 1) * ONES)) << LO);
+    }
+}
+template <int BL, int L, int Z = 0>
+__device__ __forceinline__ void digit_words(const u32 (&s)[3], const u32 (&e)[3], u32 *d)
+{
+    if constexpr (Z < L) {
+        constexpr u32 ONES = 0x01010101u, BIAS = 0x80 * ONES;  // keeps the bytes' differences from borrowing
+        d[Z] = (field4<BL * Z, BL>(s) + (BIAS - ((1u << (BL - 1)) - 1) * ONES) - field4<BL * Z, 1>(e)) ^ BIAS;
+        digit_words<BL, L, Z + 1>(s, e, d);
+    }
+}
+
+// Digits of 32 ciphertexts x 128 coefficients, the operand's layout being [row
+// tile][K block][level][half][128 rows][16 bytes].  In shared memory row r of run
+// g (K block, half) lies at r ^ g: the eight runs of a warp's words would
+// otherwise meet in the same banks.  Bound: the integer ALU, 24 instructions per
+// coefficient (26 us per 3584 rows; digit by digit, 50 and six byte stores, 37).
+constexpr int DR = 32;
 template <int BL, int L, bool GEN>
 __global__ void __launch_bounds__(256) digits_kernel(const u64 *__restrict__ in, uint8_t *__restrict__ dig, u32 B)
 {
-    __shared__ __align__(16) uint8_t sm[L * A_STEP];
-    const u32 blk = blockIdx.x, tile = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll 4
-    for (u32 r = warp; r < (u32)TM; r += 8) {
-        const u32 c = tile * TM + r;
-        int d[L];
-        ks_decomp<BL, L, GEN>(c < B ? in[(size_t)c * (N + 1) + blk * YB + lane] : 0ull, d);
+    __shared__ __align__(16) u32 sm[4 * L * 2 * DR * 4];  // [K block][level][half][row][4 words]
+    const u32 run = blockIdx.x, row0 = blockIdx.y * DR, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const u32 g = lane >> 2;
 #pragma unroll
-        for (int z = 0; z < L; z++) sm[z * A_STEP + (lane >> 4) * (TM * 16) + r * 16 + (lane & 15)] = (uint8_t)d[z];
+    for (u32 k = 0; k < DR / 8; k++) {
+        const u32 r = warp + 8 * k, c = row0 + r;
+        u32 s[4], e[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const u32 hi = c < B ? reinterpret_cast<const u32 *>(in)[2 * ((size_t)c * (N + 1) + run * 128 + 32 * j + lane) + 1] : 0u;
+            digit_fields<BL, L, GEN>(hi, s[j], e[j]);
+        }
+        u32 ts[3], te[3], d[L];
+        transpose(s, ts);
+        transpose(e, te);
+        digit_words<BL, L>(ts, te, d);
+#pragma unroll
+        for (int z = 0; z < L; z++) sm[((((g >> 1) * L + z) * 2 + (g & 1)) * DR + (r ^ g)) * 4 + (lane & 3)] = d[z];
     }
     __syncthreads();
-    uint4 *dst = reinterpret_cast<uint4 *>(dig + ((size_t)tile * NBLK + blk) * (L * A_STEP));
-    for (u32 i = threadIdx.x; i < L * A_STEP / 16; i += 256) dst[i] = reinterpret_cast<const uint4 *>(sm)[i];
+    // runs of 32 rows x 16 bytes
+    uint8_t *dst = dig + ((size_t)(row0 / TM) * NBLK + run * 4) * (L * A_STEP) + (row0 % TM) * 16;
+    for (u32 i = threadIdx.x; i < 4 * L * 2 * DR; i += 256) {
+        const u32 r = i % DR, half = i / DR % 2, z = i / (2 * DR) % L, blk = i / (2 * DR * L);
+        *reinterpret_cast<uint4 *>(dst + (blk * L + z) * A_STEP + half * (TM * 16) + r * 16) =
+            reinterpret_cast<const uint4 *>(sm)[i - r + (r ^ (blk * 2 + half))];
+    }
 }
 
-// KSK [x][coefficient][level] -> column tiles of 85 outputs, [tile][block of 32
-// coefficients][level][half][column 3 (x mod 85) + byte][16 coefficients]; the
-// last column of a tile stays zero
+// KSK [x][coefficient][level] -> column tiles of 85 outputs, [tile][K block]
+// [level][half][column 3 (x mod 85) + byte][16 coefficients, in the order of
+// k_coef]; the last column of a tile stays zero
 __global__ void __launch_bounds__(256) layout_kernel(const u32 *__restrict__ ksk, uint8_t *__restrict__ dst, u32 n, u32 L)
 {
     const u32 i = blockIdx.x * 256 + threadIdx.x, per_x = N / 16 * L;
     if (i >= (n + 1) * per_x) return;
     const u32 x = i / per_x, y16 = i % per_x / L, z = i % L;
-    const u32 *src = ksk + ((size_t)x * N + y16 * 16) * L + z;
+    const u32 *src = ksk + (size_t)x * N * L + z;
     u32 w[3][4];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         w[0][j] = w[1][j] = w[2][j] = 0;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            const u32 v = src[(4 * j + k) * L] & ((1u << KS_W) - 1);
+            const u32 v = src[k_coef(y16 / 2, (y16 & 1) * 16 + 4 * j + k) * L] & ((1u << KS_W) - 1);
 #pragma unroll
             for (int b = 0; b < 3; b++) w[b][j] |= ((v >> (8 * b)) & 0xFF) << (8 * k);
         }
@@ -275,7 +353,7 @@ cudaError_t kstc_set_attributes()
 template <bool GEN>
 static cudaError_t launch_digits(const uint64_t *in, uint8_t *dig, u32 B, uint32_t bl, uint32_t L, cudaStream_t s)
 {
-    const dim3 grid(kstc::NBLK, (B + kstc::TM - 1) / kstc::TM);
+    const dim3 grid(N / 128, (B + kstc::DR - 1) / kstc::DR);
     if (bl == 3 && L == 6) kstc::digits_kernel<3, 6, GEN><<<grid, 256, 0, s>>>(in, dig, B);
     else if (bl == 3 && L == 5) kstc::digits_kernel<3, 5, GEN><<<grid, 256, 0, s>>>(in, dig, B);
     else if (bl == 2 && L == 8) kstc::digits_kernel<2, 8, GEN><<<grid, 256, 0, s>>>(in, dig, B);
