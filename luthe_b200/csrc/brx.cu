@@ -224,11 +224,12 @@ __device__ __forceinline__ void give_up(Ctl *ctl, u32 *sync)
     *(volatile u32 *)&ctl->failed = 1;
     atomicExch(sync, 1u);
 }
-// Bounded waits: by the device-wide number of polls and by about two seconds
-// (counted in 2^10 clocks).  They return false once the CTA has given up, so
-// that after a wait ran out anywhere every role runs to its end without
-// blocking.
-constexpr u32 WAIT_KCLOCKS = 4000000;
+// Bounded waits: by the device-wide number of polls (times 32, these polls being
+// short) and by about half a minute (counted in 2^10 clocks): CTAs of a launch
+// may start late, when other work holds their SMs.  They return false once the
+// CTA has given up, so that after a wait ran out anywhere every role runs to its
+// end without blocking.
+constexpr u32 WAIT_KCLOCKS = 60000000;
 struct Patience {
     u32 left = WAIT_KCLOCKS, last = (u32)clock();
     // asked every few polls: has this wait lasted too long, or the CTA given up?
@@ -384,7 +385,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     Ctl *ctl = reinterpret_cast<Ctl *>(sm + SM_CTL);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const u32 smem = tc::smem_u32(sm);
-    const u32 polls = (u32)min(*polls_p, 0xFFFFFFFFull);
+    const u32 polls = (u32)min(min(*polls_p, 1ull << 32) * 32, 0xFFFFFFFFull);
 
     if (tid == 0) {
         for (int i = 0; i < STAGES; i++) {

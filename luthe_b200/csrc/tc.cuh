@@ -156,12 +156,6 @@ __device__ __forceinline__ u64 mad_wide(u32 a, u32 b, u64 c)
     asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
     return r;
 }
-__device__ __forceinline__ u64 mad_wide_s(u32 a, u32 b, u64 c)
-{
-    u64 r;
-    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
-    return r;
-}
 // Two residues lo + hi 2^32 mod p (lazy), lo, hi < 2^51.  With hi = h1:h0 and
 // 2^64 = 2^32 - 1 each is t + h0 2^32, t = lo + h1 (2^32 - 1); the sum leaves
 // 64 bits only when h0 is within t_hi < 2^21 of 2^32, so that case is a branch
