@@ -32,6 +32,12 @@ METRIC = "KS+PBS bootstraps/s on 1 B200, batched vs plain, bit-exact; p50/p99 op
 UNIT = "bootstraps/s"
 MODMUL_PER_BOOTSTRAP = 804 * 53248          # 4 NTT-class transforms + BSK MAC per BR step
 IMAD_PER_MODMUL = 4                         # 64x64->128 product as 4 32-bit IMAD
+# 8-bit multiply-adds of one bootstrap's blind rotation on the tensor cores, per step: forward and inverse
+# transforms (64 rows x 512 columns x 192 and x 256 bytes), products (64 points x 2 columns x 256 x 512)
+MAC8_PER_BOOTSTRAP = 804 * (64 * 512 * (192 + 256) + 64 * 2 * 256 * 512)
+MAC8_PER_CLOCK = 8192                       # a 128 x 256 x 32 tcgen05 kind::i8 takes 128 clocks (timed) on one SM
+BR_WAVE = 592                               # ciphertexts of one tensor-core blind-rotation launch
+KS_PASS, KS_SPLIT_MAX = 3584, 1024          # ciphertexts of one key-switch pass; largest pass that splits K
 KS_MAC_PER_BOOTSTRAP = 2048 * 6 * 805
 L2_FLUSH_BYTES = 256 << 20
 
@@ -50,9 +56,9 @@ def parse():
     ap.add_argument("--no-autotune", action="store_true",
                     help="keep the default launch shape (profiling runs: no tuning trials among the launches)")
     ap.add_argument("--ncu-case", nargs="?", const="pbs", choices=("pbs", "other", "plain"),
-                    help="small profiling case, then exit: 'pbs' (default) KS+PBS of 296 BLWEs (one persistent "
-                         "wave), twice; 'other' the NTT product of 4096 pairs and the key switch of 16384 BLWEs, once "
-                         "each; 'plain' KS+PBS of one BLWE (the 2-SM latency form), twice")
+                    help="small profiling case, then exit: 'pbs' (default) KS+PBS of 296 BLWEs (one couple "
+                         "of ciphertexts per SM), twice; 'other' the NTT product of 4096 pairs and the key switch of 16384 BLWEs, once "
+                         "each; 'plain' KS+PBS of one BLWE (the 8-SM latency form), twice")
     return ap.parse_args()
 
 
@@ -107,9 +113,9 @@ class Clocks:
 
 def ncu_record():
     """The ncu figures of the blind-rotation kernel kept in
-    profiles/br_kernel_ncu.json (written from an ncu capture; it names the
+    profiles/brx_kernel_ncu.json (written from an ncu capture; it names the
     commit and the command it was captured with), or None."""
-    path = os.path.join(ROOT, "profiles", "br_kernel_ncu.json")
+    path = os.path.join(ROOT, "profiles", "brx_kernel_ncu.json")
     try:
         with open(path) as f:
             return json.load(f)
@@ -385,8 +391,8 @@ def hbm_peak_gbs():
 
 
 def br_launches_per_step(B, nsm, g, tail_max=None):
-    """Blind-rotation launches of one KS+PBS call (luthe_b200/csrc/kernels.cu,
-    launch_blind_rotate): one, or two when a partial last wave of at most
+    """Butterfly blind-rotation launches of one KS+PBS call of a context without
+    the tensor-core form (luthe_b200/csrc/kernels.cu, launch_blind_rotate): one, or two when a partial last wave of at most
     tail_max ciphertexts (default: the SM count) is split off into its own
     launch."""
     wave = nsm * g
@@ -395,24 +401,35 @@ def br_launches_per_step(B, nsm, g, tail_max=None):
     return 2 if (g > 1 and B > wave and 0 < tail <= tail_max) else 1
 
 
+def launches_per_step(B, nsm):
+    """Kernel launches of one KS+PBS call (luthe_b200/csrc/api.cu and ks_tc.cu):
+    per key-switch pass the digits, the product and, where K is split, the sum
+    of the parts; one blind rotation per BR_WAVE ciphertexts or remainder."""
+    ks = 0
+    for done in range(0, B, KS_PASS):
+        m = min(KS_PASS, B - done)
+        tiles = (804 // 85 + 1) * ((m + 255) // 256)
+        ks += 3 if m <= KS_SPLIT_MAX and nsm // tiles > 1 else 2
+    return ks + (B + BR_WAVE - 1) // BR_WAVE
+
+
 def config_dict():
     return {
         "workload": "batched KS+PBS of uneven batches 1+17+256+1000+4096 = 5370 BLWEs in one call, "
                     "each batch its own random 4-bit LUT; TFHE n=804 k=1 N=2048 PBS 23x1 KS 3x6 mod 2^21, "
                     "NTT mod 2^64-2^32+1",
-        "launch": "one CUDA graph per step (luthe_ks_pbs_graph): key switch + persistent blind rotation "
-                  "(+ a tail launch when the last wave is partial)",
+        "launch": "one CUDA graph per step (luthe_ks_pbs_graph): key switch + blind rotation in launches "
+                  "of 592 ciphertexts and a remainder",
         "batches": BATCHES, "ciphertexts_per_step": sum(BATCHES),
-        "l2": "flushed between timed steps (256 MiB device write); BSK 52.7 MB and KSK 44 MB are L2-resident "
-              "by design inside a step",
+        "l2": "flushed between timed steps (256 MiB device write); the expanded BSK (2 MB per LWE coefficient) "
+              "is read once per launch, inputs and outputs 88 MB each",
         "parallelism": "replicas (one independent engine per GPU, no collective on the data path)",
     }
 
 
 def ncu_case(B=296):
-    """KS+PBS of B identity-LUT BLWEs twice (296: one persistent wave, the case
-    the blind-rotation ncu summaries under profiles/ are captured on; 1: the
-    plain path), checked by decryption."""
+    """KS+PBS of B identity-LUT BLWEs twice (296: one couple of ciphertexts
+    per SM; 1: the plain path), checked by decryption."""
     import torch
     import luthe_b200 as L
     p = L.default_params()
@@ -555,7 +572,9 @@ def main():
         br_ms.append(e0.elapsed_time(e1))
     br_s = statistics.median(br_ms) * 1e-3
     imad_peak, glmul_peak = L.measure_int_peak(local)
-    achieved_imad = B * MODMUL_PER_BOOTSTRAP * IMAD_PER_MODMUL / br_s
+    nsm = torch.cuda.get_device_properties(local).multi_processor_count
+    mac8_peak = nsm * MAC8_PER_CLOCK * 1e6 * (clk["sm_mhz"] or clk["sm_max_mhz"] or 1965.0)
+    mac8 = B * MAC8_PER_BOOTSTRAP / br_s
     ncu = ncu_record()
     traffic, traffic_how = read_traffic(B, ncu)
 
@@ -633,7 +652,7 @@ def main():
         "keyswitch_16384": {
             "ms": ks_ms, "ciphertexts_per_s": 16384 / (ks_ms * 1e-3),
             "mac_per_s": 16384 * KS_MAC_PER_BOOTSTRAP / (ks_ms * 1e-3),
-            "imad_frac_of_measured_peak": 16384 * KS_MAC_PER_BOOTSTRAP / (ks_ms * 1e-3) / imad_peak,
+            "mac8_frac": 16384 * KS_MAC_PER_BOOTSTRAP * 3 / (ks_ms * 1e-3) / mac8_peak,  # three KSK bytes
             "note": "16384 BLWEs of dimension 2048 -> n=804, KSK 3x6 mod 2^21"},
     }
 
@@ -690,11 +709,8 @@ def main():
         cpu["bit_exact_all"] = f"{eq}/{B}"
         cpu["bit_exact_all_s"] = round(time.perf_counter() - t0, 1)
 
-    # our kernels inside the timed region: per step one key switch and one or
-    # two blind-rotation launches
-    nsm = torch.cuda.get_device_properties(local).multi_processor_count
-    chosen = tune.get("chosen") or {}
-    launches = args.steps * (1 + br_launches_per_step(B, nsm, chosen.get("cts_per_cta", 2), chosen.get("tail_max")))
+    # our kernels inside the timed region
+    launches = args.steps * launches_per_step(B, nsm)
 
     if rank == 0:
         q = lambda xs, p: float(np.percentile(xs, p))
@@ -707,11 +723,11 @@ def main():
                            "plain_p50": q(plain_ms, 50), "plain_p99": q(plain_ms, 99)},
             "plain_bootstraps_per_s": 1e3 / statistics.mean(plain_ms),
             "batched_over_plain": value / world / (1e3 / statistics.mean(plain_ms)),
-            "roofline": {"bound": "int", "kernel": "br_kernel", "achieved": achieved_imad / 1e12,
-                         "peak": imad_peak / 1e12, "unit": "TIMAD/s", "frac": achieved_imad / imad_peak,
-                         "peak_source": "measured live (luthe_measure_int_peak, 32-bit IMAD probe)",
-                         "work": f"{MODMUL_PER_BOOTSTRAP} modmul x {IMAD_PER_MODMUL} IMAD per bootstrap",
-                         "traffic": traffic, "traffic_unit": f"DRAM bytes per launch ({traffic_how})",
+            "roofline": {"bound": "int8 tensor", "kernel": "brx_kernel", "achieved": mac8 / 1e12,
+                         "peak": mac8_peak / 1e12, "unit": "TMAC/s (8-bit)", "frac": mac8 / mac8_peak,
+                         "peak_source": f"{MAC8_PER_CLOCK} MACs a clock and SM (kind::i8, timed) at the SM clock under load",
+                         "work": f"{MAC8_PER_BOOTSTRAP} 8-bit MACs per bootstrap",
+                         "traffic": traffic, "traffic_unit": f"DRAM bytes per step ({traffic_how})",
                          "modmul_frac": B * MODMUL_PER_BOOTSTRAP / br_s / glmul_peak,
                          "glmul_peak_per_s": glmul_peak, "br_ms": br_s * 1e3,
                          "ncu": ncu and {k: ncu.get(k) for k in ("commit", "kernel", "command", "pipes", "l2",
