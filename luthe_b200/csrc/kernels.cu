@@ -1090,10 +1090,12 @@ cudaError_t br_set_attributes(const BrConfig &cfg, uint32_t n)
     }
 }
 
-cudaError_t br_cluster_limits(BrConfig *cfg)
+void br_cluster_limits(BrConfig *cfg)
 {
-    cudaError_t e = parts::prepare(4, &cfg->oct_max);
-    return e == cudaSuccess ? parts::prepare(2, &cfg->quad_max) : e;
+    // a device (or a share of one) that cannot place such clusters does without
+    if (parts::prepare(4, &cfg->oct_max) != cudaSuccess) cfg->oct_max = 0;
+    if (parts::prepare(2, &cfg->quad_max) != cudaSuccess) cfg->quad_max = 0;
+    cudaGetLastError();
 }
 
 // One blind-rotation launch.  G: ciphertexts per CTA (1 or 2, br_kernel);

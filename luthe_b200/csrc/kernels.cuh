@@ -94,7 +94,7 @@ cudaError_t launch_blind_rotate(const BrConfig &cfg, int num_sms, const uint32_t
                                 size_t *main_count = nullptr);
 size_t br_smem_bytes(const BrConfig &cfg, uint32_t n);
 cudaError_t br_set_attributes(const BrConfig &cfg, uint32_t n);
-cudaError_t br_cluster_limits(BrConfig *cfg);  // sets oct_max and quad_max for the current device
+void br_cluster_limits(BrConfig *cfg);  // sets oct_max and quad_max for the current device
 
 enum LweOp : int { LWE_ADD = 0, LWE_SUB = 1, LWE_MAC = 2, LWE_ADDS = 3, LWE_SUBS = 4, LWE_SSUB = 5, LWE_MULS = 6 };
 // one linear DOp or register copy (op = LWE_COPY) on slots of a BLWE pool
