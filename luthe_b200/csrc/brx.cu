@@ -743,7 +743,8 @@ __global__ void __launch_bounds__(THREADS, 1)
         bool good = true;
         const u32 tiles = (B + TILE - 1) / TILE;
         u32 seq = 0;  // couples so far
-        // each lane watches one tile's counter; false if that wait ran out
+        // each lane watches one tile's counter; false if that wait ran out.  The barrier after the vote orders what
+        // the watching lane acquired before the copies that lane 0 issues: the vote alone orders no memory.
         auto wait_tile = [&](u32 tile, u32 &complete, bool units, u32 i) {
             Patience patience;
             for (u32 it = 0; !(complete >> tile & 1); it++) {
@@ -756,6 +757,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     return false;
                 }
             }
+            __syncwarp();
             return true;
         };
         for (u32 i = 0; i <= n && good; i++) {
