@@ -108,8 +108,7 @@ void drop_graphs(luthe_ctx *c)
 static size_t brx_bytes(const luthe_ctx *c)
 {
     using namespace brx;
-    return (size_t)c->p.lwe_dim * STEP_BYTES + WEIGHT_BYTES + (EVAL_WORDS + PROD_WORDS + ACC_WORDS) * 8 +
-           SYNC_BYTES;
+    return (size_t)c->p.lwe_dim * STEP_BYTES + WEIGHT_BYTES + 2 * BUFFER_BYTES;
 }
 
 static void brx_release(luthe_ctx *c)
@@ -117,7 +116,7 @@ static void brx_release(luthe_ctx *c)
     if (!c->ws.weights || c->ws_held) return;
     drop_graphs(c);  // captured launches use the workspace
     cudaFree(c->ws.weights);  // one allocation
-    c->ws = brx::Workspace{};
+    c->ws = c->ws_cap = brx::Workspace{};
     c->used -= brx_bytes(c);
 }
 
@@ -137,24 +136,28 @@ static int brx_prepare(luthe_ctx *c, const uint64_t *d_std)
             cudaGetLastError();
             return LUTHE_OK;
         }
-        Workspace w;
-        w.bsk = base + WEIGHT_BYTES;
-        w.eval = (uint64_t *)(w.bsk + (size_t)c->p.lwe_dim * STEP_BYTES);
-        w.prod = w.eval + EVAL_WORDS;
-        w.acc = w.prod + PROD_WORDS;
-        w.sync = (uint32_t *)(w.acc + ACC_WORDS);
-        w.weights = base;
+        Workspace w[2];
+        cudaError_t e = cudaSuccess;
+        for (int k = 0; k < 2 && e == cudaSuccess; k++) {
+            w[k].weights = base;
+            w[k].bsk = base + WEIGHT_BYTES;
+            w[k].eval = (uint64_t *)(w[k].bsk + (size_t)c->p.lwe_dim * STEP_BYTES + k * BUFFER_BYTES);
+            w[k].prod = w[k].eval + EVAL_WORDS;
+            w[k].acc = w[k].prod + PROD_WORDS;
+            w[k].sync = (uint32_t *)(w[k].acc + ACC_WORDS);
+            e = slab_wait_polls_address(&w[k].polls);
+            if (e == cudaSuccess) e = make_prod_map(w[k]);
+        }
         std::vector<uint8_t> host(WEIGHT_BYTES);
         build_weights(host.data());
-        cudaError_t e = slab_wait_polls_address(&w.polls);
         if (e == cudaSuccess) e = set_attributes();
-        if (e == cudaSuccess) e = make_prod_map(w);
         if (e == cudaSuccess) e = cudaMemcpy(base, host.data(), host.size(), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) {
             cudaFree(base);
             return fail(LUTHE_E_CUDA, "blind rotation setup: %s", cudaGetErrorString(e));
         }
-        c->ws = w;
+        c->ws = w[0];
+        c->ws_cap = w[1];
         c->used += bytes;
     }
     CUDA_TRY(launch_expand(d_std, c->ws, c->p.lwe_dim, 0));
@@ -168,7 +171,7 @@ static void kstc_release(luthe_ctx *c)
     if (!c->kt.ksk || c->kt_held) return;
     drop_graphs(c);
     cudaFree(c->kt.ksk);  // one allocation
-    c->kt = KsTc{};
+    c->kt = c->kt_cap = KsTc{};
     c->used -= c->kt_bytes;
     c->kt_bytes = 0;
 }
@@ -183,18 +186,20 @@ static int kstc_prepare(luthe_ctx *c, const uint32_t *d_raw)
     if (!c->kt.ksk) {
         const size_t ksk = kstc_ksk_bytes(n, L), part = KSTC_PART_ROWS * (size_t)c->xpad * 4;
         size_t rows = 3584;
-        while (rows >= 256 && over_budget(c, ksk + part + kstc_digit_bytes(rows, L))) rows /= 2;
+        while (rows >= 256 && over_budget(c, ksk + 2 * (part + kstc_digit_bytes(rows, L)))) rows /= 2;
         if (rows < 256) return LUTHE_OK;
-        const size_t bytes = ksk + part + kstc_digit_bytes(rows, L);
+        const size_t set = part + kstc_digit_bytes(rows, L), bytes = ksk + 2 * set;
         uint8_t *base = nullptr;
         if (cudaMalloc((void **)&base, bytes) != cudaSuccess) {
             cudaGetLastError();
             return LUTHE_OK;
         }
         c->kt = KsTc{base, base + ksk + part, (uint32_t *)(base + ksk), rows};
+        c->kt_cap = KsTc{base, c->kt.dig + set, (uint32_t *)(base + ksk + set), rows};
         c->kt_bytes = bytes;
         c->used += bytes;
         CUDA_TRY(cudaMemset(c->kt.part, 0, part));
+        CUDA_TRY(cudaMemset(c->kt_cap.part, 0, part));
         CUDA_TRY(kstc_set_attributes());
     }
     CUDA_TRY(launch_kstc_layout(d_raw, c->kt.ksk, n, L, 0));
@@ -230,6 +235,8 @@ extern "C" int luthe_ctx_create(const luthe_params *p, int device, uint64_t budg
     if (e == cudaSuccess) e = br_set_attributes(BrConfig{1, 1}, p->lwe_dim);
     if (e == cudaSuccess) e = br_set_attributes(BrConfig{2, 1}, p->lwe_dim);
     if (e == cudaSuccess) br_cluster_limits(&c->br);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ws_done, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->kt_done, cudaEventDisableTiming);
     if (e == cudaSuccess) {
         // diagnostics: LUTHE_SLAB_WAIT_POLLS bounds each BSK-slab wait (0: run out at once)
         const char *polls = getenv("LUTHE_SLAB_WAIT_POLLS");
@@ -268,6 +275,8 @@ extern "C" void luthe_ctx_destroy(luthe_ctx *c)
     dfree(c, c->d_hids, c->hcap * 4);
     if (c->ev_main) cudaEventDestroy(c->ev_main);
     if (c->ev_in) cudaEventDestroy(c->ev_in);
+    if (c->ws_done) cudaEventDestroy(c->ws_done);
+    if (c->kt_done) cudaEventDestroy(c->kt_done);
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
     delete c;
 }
@@ -441,16 +450,31 @@ int need_keys(luthe_ctx *c)
     return LUTHE_OK;
 }
 
-// A launch that the caller captures may be replayed whenever they like: what it
-// uses is held.  (The context's own graphs are dropped with what they use.)
-static bool captured(luthe_ctx *c, cudaStream_t s)
+// Who runs a launch enqueued on stream s.  CALLER: it is captured by the caller,
+// who may replay it whenever they like: what it uses is held, and its buffers
+// are those of captured launches.  OWN: captured by luthe_ks_pbs_graph; the
+// context drops its graphs with what they use, and their launches take turns.
+enum class Run { NOW, OWN, CALLER };
+static Run run_of(luthe_ctx *c, cudaStream_t s)
 {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
         cudaGetLastError();  // the launch itself reports it
-        return false;
+        return Run::NOW;
     }
-    return st == cudaStreamCaptureStatusActive && !c->own_capture;
+    return st != cudaStreamCaptureStatusActive ? Run::NOW : c->own_capture ? Run::OWN : Run::CALLER;
+}
+// What `enqueue` puts on stream s runs after the last work that `done` was
+// recorded behind, and `done` then stands for it: streams that the caller left
+// unordered cannot meet in the buffers.  (One context, one thread: luthe.h.)
+template <typename F>
+static cudaError_t in_turn(cudaEvent_t done, cudaStream_t s, F enqueue)
+{
+    cudaError_t e = cudaStreamWaitEvent(s, done, 0);
+    if (e != cudaSuccess) return e;
+    e = enqueue();
+    const cudaError_t r = cudaEventRecord(done, s);  // after an error too: part of the work may run
+    return e != cudaSuccess ? e : r;
 }
 
 // Blind rotation of a whole batch on stream s.  Batches above one ciphertext
@@ -470,26 +494,32 @@ static cudaError_t enqueue_blind_rotate(luthe_ctx *c, const uint32_t *d_l2n, con
         return launch_blind_rotate(c->br, c->nsm, d_l2n, c->d_luts, d_ids, c->nlut, c->d_bsk, c->d_tw, d_out, count, n,
                                    c->d_err, s, nullptr, mlk, c->p.pbs_base_log, c->tie_rule, main_done, main_count);
     if (main_count) *main_count = count;
-    c->ws_held |= captured(c, s);
-    for (size_t done = 0; done < count;) {
-        const size_t left = count - done, take = std::min(left, brx::WAVE);
-        if (done && main_done && take == left) {
-            cudaError_t e = cudaEventRecord(main_done, s);
+    const Run run = run_of(c, s);
+    const brx::Workspace &ws = run == Run::CALLER ? c->ws_cap : c->ws;
+    auto launches = [&]() -> cudaError_t {
+        for (size_t done = 0; done < count;) {
+            const size_t left = count - done, take = std::min(left, brx::WAVE);
+            if (done && main_done && take == left) {
+                cudaError_t e = cudaEventRecord(main_done, s);
+                if (e != cudaSuccess) return e;
+                if (main_count) *main_count = done;
+            }
+            const uint32_t *l2n = d_l2n + done * (n + 1), *ids = d_ids + done;
+            uint64_t *out = d_out + done * mlk * (size_t)(N + 1);
+            cudaError_t e =
+                take <= (size_t)c->nsm
+                    ? launch_blind_rotate(c->br, c->nsm, l2n, c->d_luts, ids, c->nlut, c->d_bsk, c->d_tw, out, take, n,
+                                          c->d_err, s, nullptr, mlk, c->p.pbs_base_log, c->tie_rule)
+                    : brx::launch(ws, c->nsm, l2n, c->d_luts, ids, c->nlut, out, take, n, c->d_err, s, mlk,
+                                  c->p.pbs_base_log, c->tie_rule);
             if (e != cudaSuccess) return e;
-            if (main_count) *main_count = done;
+            done += take;
         }
-        const uint32_t *l2n = d_l2n + done * (n + 1), *ids = d_ids + done;
-        uint64_t *out = d_out + done * mlk * (size_t)(N + 1);
-        cudaError_t e =
-            take <= (size_t)c->nsm
-                ? launch_blind_rotate(c->br, c->nsm, l2n, c->d_luts, ids, c->nlut, c->d_bsk, c->d_tw, out, take, n,
-                                      c->d_err, s, nullptr, mlk, c->p.pbs_base_log, c->tie_rule)
-                : brx::launch(c->ws, c->nsm, l2n, c->d_luts, ids, c->nlut, out, take, n, c->d_err, s, mlk,
-                              c->p.pbs_base_log, c->tie_rule);
-        if (e != cudaSuccess) return e;
-        done += take;
-    }
-    return cudaSuccess;
+        return cudaSuccess;
+    };
+    if (run == Run::NOW) return in_turn(c->ws_done, s, launches);
+    c->ws_held |= run == Run::CALLER;
+    return launches();
 }
 
 // Key switch of a batch on stream s: on the tensor cores at every size (one
@@ -500,9 +530,14 @@ static cudaError_t enqueue_keyswitch(luthe_ctx *c, const uint64_t *d_in, uint32_
                                      size_t count, cudaStream_t s, uint32_t *d_part)
 {
     if (c->kt.ksk) {
-        c->kt_held |= captured(c, s);
-        return launch_keyswitch_tc(c->kt, c->nsm, d_in, d_out21, d_out2N, count, c->p.lwe_dim, c->xpad, c->p.ks_base_log,
-                                   c->p.ks_level, c->tie_rule, c->d_err, s);
+        const Run run = run_of(c, s);
+        auto launches = [&] {
+            return launch_keyswitch_tc(run == Run::CALLER ? c->kt_cap : c->kt, c->nsm, d_in, d_out21, d_out2N, count,
+                                       c->p.lwe_dim, c->xpad, c->p.ks_base_log, c->p.ks_level, c->tie_rule, c->d_err, s);
+        };
+        if (run == Run::NOW) return in_turn(c->kt_done, s, launches);
+        c->kt_held |= run == Run::CALLER;
+        return launches();
     }
     return launch_keyswitch(d_in, c->d_ksk, d_out21, d_out2N, count, c->p.lwe_dim, c->xpad, s, nullptr, c->p.ks_base_log,
                             c->p.ks_level, c->tie_rule, d_part);
@@ -544,6 +579,15 @@ extern "C" int luthe_ks_pbs_ml(luthe_ctx *c, const uint64_t *d_in, const uint32_
     return LUTHE_OK;
 }
 
+static cudaError_t launch_own_graph(luthe_ctx *c, const GraphEntry &g)
+{
+    auto launch = [&] { return cudaGraphLaunch(g.exec, g.stream); };
+    auto rotation = [&] {
+        return c->ws.bsk && g.count > (size_t)c->nsm ? in_turn(c->ws_done, g.stream, launch) : launch();
+    };
+    return c->kt.ksk ? in_turn(c->kt_done, g.stream, rotation) : rotation();
+}
+
 extern "C" int luthe_ks_pbs_graph(luthe_ctx *c, const uint64_t *d_in, const uint32_t *d_ids, uint64_t *d_out,
                                   size_t count, void *stream)
 {
@@ -557,7 +601,7 @@ extern "C" int luthe_ks_pbs_graph(luthe_ctx *c, const uint64_t *d_in, const uint
     if ((r = ensure_scratch(c, count))) return r;
     for (auto &g : c->graphs)
         if (g.in == d_in && g.ids == d_ids && g.out == d_out && g.count == count && g.stream == s) {
-            CUDA_TRY(cudaGraphLaunch(g.exec, s));
+            CUDA_TRY(launch_own_graph(c, g));
             return LUTHE_OK;
         }
     cudaGraph_t graph;
@@ -577,7 +621,7 @@ extern "C" int luthe_ks_pbs_graph(luthe_ctx *c, const uint64_t *d_in, const uint
         c->graphs.erase(c->graphs.begin());
     }
     c->graphs.push_back(GraphEntry{d_in, d_ids, d_out, count, s, exec});
-    CUDA_TRY(cudaGraphLaunch(exec, s));
+    CUDA_TRY(launch_own_graph(c, c->graphs.back()));
     return LUTHE_OK;
 }
 

@@ -26,6 +26,7 @@ struct alignas(64) TensorMap {  // CUtensorMap
     uint64_t opaque[16];
 };
 
+// Launches that overlap on the GPU must not share eval, prod, acc and sync.
 struct Workspace {
     uint8_t *weights = nullptr;   // [WF][WI][roots]
     uint8_t *bsk = nullptr;       // [n][PK][col][row][BLOCK_BYTES]
@@ -38,6 +39,7 @@ struct Workspace {
 };
 constexpr size_t EVAL_WORDS = TILES * TILE_WORDS, PROD_WORDS = EVAL_WORDS, ACC_WORDS = EVAL_WORDS;
 constexpr size_t SYNC_BYTES = 128 * (1 + 2 * TILES);
+constexpr size_t BUFFER_BYTES = (EVAL_WORDS + PROD_WORDS + ACC_WORDS) * 8 + SYNC_BYTES;  // 63 MB: what a launch writes
 
 void build_weights(uint8_t *host /* WEIGHT_BYTES */);
 cudaError_t set_attributes();

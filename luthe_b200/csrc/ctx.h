@@ -40,8 +40,12 @@ struct luthe_ctx {
     cudaEvent_t ev_in = nullptr;         // host path: a chunk of inputs has landed
     luthe::BrConfig br{2, 1};
     uint32_t tie_rule = luthe::TIE_RTL;  // decomposition tie rule (luthe_set_tie_rule)
-    luthe::brx::Workspace ws;            // tensor-core blind rotation; ws.bsk null: not available
-    luthe::KsTc kt;                      // tensor-core key switch; kt.ksk null: not available
+    // tensor-core blind rotation (ws.bsk null: not available) and key switch (kt.ksk null): the keys, and two sets of
+    // buffers, for the context's calls, which take turns at them whatever streams they run on (ws_done, kt_done: the
+    // last one's work), and for launches that the caller captures, whose replays the context does not see
+    luthe::brx::Workspace ws, ws_cap;
+    luthe::KsTc kt, kt_cap;
+    cudaEvent_t ws_done = nullptr, kt_done = nullptr;
     size_t kt_bytes = 0;
     bool ws_held = false, kt_held = false;  // used by launches that the caller captured
     bool own_capture = false;               // a graph of luthe_ks_pbs_graph is being captured
