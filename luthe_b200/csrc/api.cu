@@ -299,6 +299,7 @@ extern "C" int luthe_upload_bsk(luthe_ctx *c, const uint64_t *h)
     if (e == cudaSuccess) r = brx_prepare(c, d_std);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     dfree(c, d_std, words * 8);
+    if (e != cudaSuccess || r) brx_release(c);
     if (e != cudaSuccess) return fail(LUTHE_E_CUDA, "BSK upload: %s", cudaGetErrorString(e));
     return r;
 }
@@ -325,8 +326,8 @@ extern "C" int luthe_upload_bsk_eval(luthe_ctx *c, const uint64_t *h)
                 }
     int r;
     if (!c->d_bsk && (r = dalloc(c, (void **)&c->d_bsk, n * SLAB_BYTES))) return r;
-    CUDA_TRY(cudaMemcpy(c->d_bsk, slab.data(), words * 8, cudaMemcpyHostToDevice));
-    // the expanded key is made from the standard domain; it must not outlive the key it was made from
+    // the expanded key is made from the standard domain; it must not outlive the key it was made from, so the
+    // memory for that copy comes before any change of the key
     uint64_t *d_std = nullptr;
     const size_t need = words * 8 + (c->ws.weights ? 0 : brx_bytes(c));
     if (c->ws_held) {  // captured launches read it: it has to follow the key
@@ -334,13 +335,15 @@ extern "C" int luthe_upload_bsk_eval(luthe_ctx *c, const uint64_t *h)
         c->used += words * 8;
     } else if (over_budget(c, need) || dalloc(c, (void **)&d_std, words * 8)) {
         brx_release(c);
-        return LUTHE_OK;
     }
-    cudaError_t e = cudaMemcpy(d_std, h, words * 8, cudaMemcpyHostToDevice);
+    cudaError_t e = cudaMemcpy(c->d_bsk, slab.data(), words * 8, cudaMemcpyHostToDevice);
+    if (!d_std) return e == cudaSuccess ? LUTHE_OK : fail(LUTHE_E_CUDA, "BSK upload: %s", cudaGetErrorString(e));
+    if (e == cudaSuccess) e = cudaMemcpy(d_std, h, words * 8, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = launch_ntt_inv(d_std, d_std, c->d_tw, n * 4, 0);
     if (e == cudaSuccess) r = brx_prepare(c, d_std);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     dfree(c, d_std, words * 8);
+    if (e != cudaSuccess || r) brx_release(c);
     if (e != cudaSuccess) return fail(LUTHE_E_CUDA, "BSK upload: %s", cudaGetErrorString(e));
     return r;
 }

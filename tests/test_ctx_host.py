@@ -52,13 +52,15 @@ class Ctx:
             assert self.upload_bsk(1) == 0 and self.upload_ksk() == 0 and self.upload_luts() == 0
 
     def upload_bsk(self, word, form="bsk"):
-        return getattr(self.lib, f"luthe_upload_{form}")(self.h, np.full(STEPS * 4 * N, word, np.uint64).ctypes.data)
+        key = np.full(STEPS * 4 * N, word, np.uint64)
+        return getattr(self.lib, f"luthe_upload_{form}")(self.h, key.ctypes.data)
 
     def upload_ksk(self):
         return self.lib.luthe_upload_ksk(self.h, self.ksk.ctypes.data)
 
     def upload_luts(self):
-        return self.lib.luthe_upload_luts(self.h, np.zeros(2 * N, np.uint64).ctypes.data, 1)
+        lut = np.zeros(2 * N, np.uint64)
+        return self.lib.luthe_upload_luts(self.h, lut.ctypes.data, 1)
 
     def call(self, name, count, stream):
         p = vp(64)
@@ -110,3 +112,26 @@ def test_captured_launches_have_buffers_of_their_own(ctx, name):
         assert ctx.call(name, 300, b) == 0
         assert ctx.call("ks_pbs_graph", 300, b) == 0
     assert ctx.lib.harness_races() == 0
+
+
+def _bsk_words(ctx):
+    w = np.zeros(2, np.uint64)
+    ctx.lib.harness_bsk_words(ctx.h, w.ctypes.data, w.ctypes.data + 8)
+    return w.tolist()
+
+
+def test_a_failed_key_upload_leaves_one_key(ctx):
+    """The two device forms of the BSK come from one key.  While captured
+    launches hold the expanded form, an evaluation-domain upload that finds no
+    memory for its copy must leave the key that was there in both."""
+    a = ctx.lib.harness_stream()
+    ctx.lib.harness_begin_capture(a)
+    assert ctx.call("ks_pbs", 300, a) == 0
+    ctx.lib.harness_end_capture(a)
+    before = _bsk_words(ctx)
+    ctx.lib.harness_fail_malloc(0, 2)
+    assert ctx.upload_bsk(2, "bsk_eval") == L.E_CUDA
+    assert _bsk_words(ctx) == before
+    assert ctx.upload_bsk(2, "bsk_eval") == 0
+    slab, expanded = _bsk_words(ctx)
+    assert slab != before[0] and expanded == 2
