@@ -121,8 +121,8 @@ static void brx_release(luthe_ctx *c)
 }
 
 // Allocate (first key) and fill the expanded key from the standard-domain BSK
-// on the device.  Without room for it the context works without: every batch
-// then runs the butterfly kernels.
+// on the device.  Where it has no room or cannot be set up the context works
+// without: every batch then runs the butterfly kernels.
 static int brx_prepare(luthe_ctx *c, const uint64_t *d_std)
 {
     using namespace brx;
@@ -153,8 +153,9 @@ static int brx_prepare(luthe_ctx *c, const uint64_t *d_std)
         if (e == cudaSuccess) e = set_attributes();
         if (e == cudaSuccess) e = cudaMemcpy(base, host.data(), host.size(), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) {
+            cudaGetLastError();
             cudaFree(base);
-            return fail(LUTHE_E_CUDA, "blind rotation setup: %s", cudaGetErrorString(e));
+            return LUTHE_OK;
         }
         c->ws = w[0];
         c->ws_cap = w[1];
@@ -177,9 +178,9 @@ static void kstc_release(luthe_ctx *c)
 }
 
 // Allocate (first key) and fill the key's form from the KSK as uploaded (d_raw,
-// on the device).  Without room every key switch runs the dp4a form.  The digit
-// buffer holds 14 row tiles of 256 (140 product CTAs at ten column tiles, one
-// wave), less where the budget is short.
+// on the device).  Without room, or where it cannot be set up, every key switch
+// runs the dp4a form.  The digit buffer holds 14 row tiles of 256 (140 product
+// CTAs at ten column tiles, one wave), less where the budget is short.
 static int kstc_prepare(luthe_ctx *c, const uint32_t *d_raw)
 {
     const uint32_t n = c->p.lwe_dim, L = c->p.ks_level;
@@ -198,9 +199,14 @@ static int kstc_prepare(luthe_ctx *c, const uint32_t *d_raw)
         c->kt_cap = KsTc{base, c->kt.dig + set, (uint32_t *)(base + ksk + set), rows};
         c->kt_bytes = bytes;
         c->used += bytes;
-        CUDA_TRY(cudaMemset(c->kt.part, 0, part));
-        CUDA_TRY(cudaMemset(c->kt_cap.part, 0, part));
-        CUDA_TRY(kstc_set_attributes());
+        cudaError_t e = cudaMemset(c->kt.part, 0, part);
+        if (e == cudaSuccess) e = cudaMemset(c->kt_cap.part, 0, part);
+        if (e == cudaSuccess) e = kstc_set_attributes();
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            kstc_release(c);
+            return LUTHE_OK;
+        }
     }
     CUDA_TRY(launch_kstc_layout(d_raw, c->kt.ksk, n, L, 0));
     return LUTHE_OK;

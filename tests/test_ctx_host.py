@@ -135,3 +135,21 @@ def test_a_failed_key_upload_leaves_one_key(ctx):
     assert ctx.upload_bsk(2, "bsk_eval") == 0
     slab, expanded = _bsk_words(ctx)
     assert slab != before[0] and expanded == 2
+
+
+def test_a_form_that_cannot_be_set_up_is_done_without(lib):
+    """The tensor-core forms are optional: where one cannot be set up, uploads
+    succeed, hold nothing for it, and calls run the other form."""
+    c = Ctx(lib, keys=False)
+    assert c.upload_luts() == 0
+    lib.harness_fail_optional(801, 801)
+    for _ in range(2):
+        assert c.upload_bsk(1) == 0 and c.upload_bsk(1, "bsk_eval") == 0 and c.upload_ksk() == 0
+    assert lib.luthe_device_bytes(c.h) < 16 << 20
+    assert c.call("ks_pbs", 300, None) == 0
+    assert c.log() == ["ks_dp4a 300", "br 300"]
+    lib.harness_fail_optional(0, 0)
+    assert c.upload_bsk(1) == 0 and c.upload_ksk() == 0
+    assert c.call("ks_pbs", 300, None) == 0
+    assert c.log() == ["ks_tc 300", "brx 300"]
+    c.close()
