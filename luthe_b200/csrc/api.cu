@@ -492,15 +492,20 @@ static cudaError_t in_turn(cudaEvent_t done, cudaStream_t s, F enqueue)
 // 13.8 ms against 20 ms of the butterfly kernels' wave (592: 21.0 ms against
 // 40), one of 100 takes 12.7 ms against 10.4 ms of the one-per-SM form (148
 // SMs, n = 804).
-// Smaller batches and remainders run the butterfly kernels.  main_done /
-// main_count as in launch_blind_rotate: the outputs before the last launch.
+// Smaller batches and remainders run the butterfly kernels, as do all batches on
+// a stream that has only some of the SMs: the tensor-core form needs a CTA on
+// each, and the clusters of eight and four SMs are counted on the whole device.
+// main_done / main_count as in launch_blind_rotate: the outputs before the last launch.
 static cudaError_t enqueue_blind_rotate(luthe_ctx *c, const uint32_t *d_l2n, const uint32_t *d_ids, uint64_t *d_out,
                                         size_t count, uint32_t mlk, cudaStream_t s, cudaEvent_t main_done = nullptr,
                                         size_t *main_count = nullptr)
 {
     const uint32_t n = c->p.lwe_dim;
-    if (!c->ws.bsk || count <= (size_t)c->nsm)
-        return launch_blind_rotate(c->br, c->nsm, d_l2n, c->d_luts, d_ids, c->nlut, c->d_bsk, c->d_tw, d_out, count, n,
+    const bool limited = brx::limited_stream(s);
+    BrConfig cfg = c->br;
+    if (limited) cfg.oct_max = cfg.quad_max = 0;
+    if (!c->ws.bsk || count <= (size_t)c->nsm || limited)
+        return launch_blind_rotate(cfg, c->nsm, d_l2n, c->d_luts, d_ids, c->nlut, c->d_bsk, c->d_tw, d_out, count, n,
                                    c->d_err, s, nullptr, mlk, c->p.pbs_base_log, c->tie_rule, main_done, main_count);
     if (main_count) *main_count = count;
     const Run run = run_of(c, s);
@@ -515,12 +520,15 @@ static cudaError_t enqueue_blind_rotate(luthe_ctx *c, const uint32_t *d_l2n, con
             }
             const uint32_t *l2n = d_l2n + done * (n + 1), *ids = d_ids + done;
             uint64_t *out = d_out + done * mlk * (size_t)(N + 1);
-            cudaError_t e =
-                take <= (size_t)c->nsm
-                    ? launch_blind_rotate(c->br, c->nsm, l2n, c->d_luts, ids, c->nlut, c->d_bsk, c->d_tw, out, take, n,
-                                          c->d_err, s, nullptr, mlk, c->p.pbs_base_log, c->tie_rule)
-                    : brx::launch(ws, c->nsm, l2n, c->d_luts, ids, c->nlut, out, take, n, c->d_err, s, mlk,
-                                  c->p.pbs_base_log, c->tie_rule);
+            cudaError_t e = cudaErrorCooperativeLaunchTooLarge;
+            if (take > (size_t)c->nsm)
+                e = brx::launch(ws, c->nsm, l2n, c->d_luts, ids, c->nlut, out, take, n, c->d_err, s, mlk,
+                                c->p.pbs_base_log, c->tie_rule);
+            if (e == cudaErrorCooperativeLaunchTooLarge) {  // a remainder, or not every SM is this process's
+                cudaGetLastError();
+                e = launch_blind_rotate(cfg, c->nsm, l2n, c->d_luts, ids, c->nlut, c->d_bsk, c->d_tw, out, take, n,
+                                        c->d_err, s, nullptr, mlk, c->p.pbs_base_log, c->tie_rule);
+            }
             if (e != cudaSuccess) return e;
             done += take;
         }

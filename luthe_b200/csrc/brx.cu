@@ -891,6 +891,22 @@ cudaError_t make_prod_map(Workspace &ws)
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+// (A cooperative launch is checked against the whole device's SMs, so that on
+// such a stream its CTAs would wait for ones that cannot start.)
+bool limited_stream(cudaStream_t s)
+{
+    using Query = decltype(&cuStreamGetGreenCtx);
+    static const Query query = [] {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        const cudaError_t e = cudaGetDriverEntryPoint("cuStreamGetGreenCtx", &fn, cudaEnableDefault, &found);
+        if (e != cudaSuccess) cudaGetLastError();
+        return e == cudaSuccess && found == cudaDriverEntryPointSuccess ? reinterpret_cast<Query>(fn) : nullptr;
+    }();  // a driver without green contexts: none
+    CUgreenCtx ctx = nullptr;
+    return query && query(s, &ctx) == CUDA_SUCCESS && ctx;
+}
+
 cudaError_t launch(const Workspace &ws, int nsm, const uint32_t *d_lwe2N, const uint64_t *d_luts,
                    const uint32_t *d_lut_id, uint32_t nlut, uint64_t *d_out, size_t B, uint32_t n, uint32_t *d_err,
                    cudaStream_t s, uint32_t mlk, uint32_t pbs_bw, uint32_t tie_rule)

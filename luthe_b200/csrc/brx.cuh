@@ -41,6 +41,8 @@ constexpr size_t EVAL_WORDS = TILES * TILE_WORDS, PROD_WORDS = EVAL_WORDS, ACC_W
 constexpr size_t SYNC_BYTES = 128 * (1 + 2 * TILES);
 constexpr size_t BUFFER_BYTES = (EVAL_WORDS + PROD_WORDS + ACC_WORDS) * 8 + SYNC_BYTES;  // 63 MB: what a launch writes
 
+// is the stream confined to some of the device's SMs (a green context's)?  launch() must not be called on one
+bool limited_stream(cudaStream_t s);
 void build_weights(uint8_t *host /* WEIGHT_BYTES */);
 cudaError_t set_attributes();
 cudaError_t make_prod_map(Workspace &ws);

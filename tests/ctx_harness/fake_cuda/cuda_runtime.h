@@ -17,7 +17,8 @@
 
 typedef int cudaError_t;
 enum {
-    cudaSuccess = 0, cudaErrorInvalidValue = 1, cudaErrorMemoryAllocation = 2, cudaErrorNotSupported = 801,
+    cudaSuccess = 0, cudaErrorInvalidValue = 1, cudaErrorMemoryAllocation = 2, cudaErrorCooperativeLaunchTooLarge = 720,
+    cudaErrorNotSupported = 801,
     cudaErrorStreamCaptureIsolation = 906, cudaErrorCapturedEvent = 907
 };
 struct fake_graph {
@@ -27,6 +28,7 @@ struct fake_stream {
     std::set<int> before;            // operations ordered before whatever comes next
     fake_graph *capture = nullptr;   // capturing into
     bool caller = false;             // ... for the caller, not for the context
+    bool limited = false;            // to some of the SMs
 };
 struct fake_event {
     std::set<int> before;

@@ -6,7 +6,7 @@
 #include "../../luthe_b200/csrc/api.cu"
 
 static std::string g_log;  // "form count;" per launch
-static int g_fail_map, g_fail_ks_attr;
+static int g_fail_map, g_fail_ks_attr, g_fail_brx;
 
 static void note(const char *form, size_t count) { g_log += std::string(form) + " " + std::to_string(count) + ";"; }
 
@@ -74,6 +74,7 @@ namespace brx {
 void build_weights(uint8_t *w) { memset(w, 0, WEIGHT_BYTES); }
 cudaError_t set_attributes() { return cudaSuccess; }
 cudaError_t make_prod_map(Workspace &) { return g_fail_map; }
+bool limited_stream(cudaStream_t s) { return fake_of(s)->limited; }
 // the expanded key's first word: that of the key it was made from
 cudaError_t launch_expand(const uint64_t *d_std, const Workspace &ws, uint32_t, cudaStream_t)
 {
@@ -83,7 +84,8 @@ cudaError_t launch_expand(const uint64_t *d_std, const Workspace &ws, uint32_t, 
 cudaError_t launch(const Workspace &ws, int, const uint32_t *, const uint64_t *, const uint32_t *, uint32_t, uint64_t *,
                    size_t B, uint32_t, uint32_t *, cudaStream_t s, uint32_t, uint32_t, uint32_t)
 {
-    note("brx", B);
+    if (g_fail_brx) return g_fail_brx;
+    note(fake_of(s)->limited ? "brx_limited" : "brx", B);
     fake_use(ws.sync, s);
     return cudaSuccess;
 }
@@ -92,6 +94,8 @@ cudaError_t launch(const Workspace &ws, int, const uint32_t *, const uint64_t *,
 
 extern "C" {
 fake_stream *harness_stream() { return new fake_stream; }
+void harness_limit(fake_stream *s) { s->limited = true; }
+void harness_fail_brx(int error) { g_fail_brx = error; }
 void harness_begin_capture(fake_stream *s)  // the caller's
 {
     s->capture = new fake_graph;
@@ -113,7 +117,7 @@ void harness_reset()
     g_fake.captured_uses.clear();
     g_fake.fail_malloc.clear();
     g_log.clear();
-    g_fail_map = g_fail_ks_attr = 0;
+    g_fail_map = g_fail_ks_attr = g_fail_brx = 0;
 }
 int harness_log(char *buf, int cap)
 {

@@ -22,6 +22,8 @@ def lib():
     h.harness_stream.restype = h.harness_end_capture.restype = vp
     h.harness_begin_capture.argtypes = h.harness_end_capture.argtypes = [vp]
     h.harness_replay.argtypes = [vp, vp]
+    h.harness_limit.argtypes = [vp]
+    h.harness_fail_brx.argtypes = [ctypes.c_int]
     h.harness_fail_malloc.argtypes = [ctypes.c_int, ctypes.c_int]
     h.harness_fail_optional.argtypes = [ctypes.c_int, ctypes.c_int]
     h.harness_bsk_words.argtypes = [vp, vp, vp]
@@ -153,3 +155,23 @@ def test_a_form_that_cannot_be_set_up_is_done_without(lib):
     assert c.call("ks_pbs", 300, None) == 0
     assert c.log() == ["ks_tc 300", "brx 300"]
     c.close()
+
+
+@pytest.mark.parametrize("name", ["blind_rotate", "ks_pbs", "ks_pbs_graph"])
+@pytest.mark.parametrize("count", [1, 20, 149, 1200])
+def test_streams_with_some_of_the_SMs(ctx, name, count):
+    """On a stream that has some of the SMs only, the tensor-core blind rotation
+    (CTAs on every SM that wait for one another) and the clusters of eight and
+    four SMs (counted on the whole device) are not launched."""
+    s = ctx.lib.harness_stream()
+    ctx.lib.harness_limit(s)
+    assert ctx.call(name, count, s) == 0
+    assert [f for f in ctx.log() if f.startswith("br")] == [f"br {count}"]
+
+
+def test_a_refused_cooperative_launch_runs_the_other_form(ctx):
+    ctx.lib.harness_fail_brx(720)
+    assert ctx.call("blind_rotate", 700, ctx.lib.harness_stream()) == 0
+    assert ctx.log() == ["br 592", "br 108"]
+    ctx.lib.harness_fail_brx(1)  # any other error is reported
+    assert ctx.call("blind_rotate", 700, ctx.lib.harness_stream()) == L.E_CUDA
