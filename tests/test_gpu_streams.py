@@ -80,3 +80,23 @@ def test_replays_beside_calls(setup, kind):
     captured.check()
     direct.check()
     del g
+
+
+def test_two_contexts(setup):
+    """Large batches of two contexts on two streams: each launch needs every SM
+    at once, and neither waits for the other's CTAs."""
+    import torch
+    keys, luts, ob = setup[1:]
+    with L.Engine(L.default_params(lwe_dim=STEPS)) as second:
+        second.upload_keys(keys)
+        second.upload_luts(luts)
+        streams = [torch.cuda.Stream() for _ in range(2)]
+        jobs = [Job((eng, keys, luts, ob), "blind_rotate", 20 + k) for k, eng in enumerate([setup[0], second] * 4)]
+        torch.cuda.synchronize()
+        for k, job in enumerate(jobs):
+            job.run(streams[k % 2])
+        torch.cuda.synchronize()
+        for eng in (setup[0], second):
+            eng.check_device_error()
+        for job in jobs:
+            job.check()
