@@ -540,9 +540,9 @@ static cudaError_t enqueue_blind_rotate(luthe_ctx *c, const uint32_t *d_l2n, con
 }
 
 // Key switch of a batch on stream s: on the tensor cores at every size (one
-// BLWE 23 us against 56 us of the split-K dp4a form, 65 of the 2x7 set 27 us
-// against 1.27 ms, 16384 of the 3x6 set 0.54 ms against 10.35: ks_tc.cu), in the dp4a form where the
-// context has no room for the tensor-core form's key.
+// BLWE 23 us against 56 us of the split-K dp4a form, 65 of the 2x7 set 24.6 us
+// against 1.24 ms, 16384 of the 3x6 set 0.55 ms against 10.35: ks_tc.cu), in the
+// dp4a form where the context has no room for the tensor-core form's key.
 static cudaError_t enqueue_keyswitch(luthe_ctx *c, const uint64_t *d_in, uint32_t *d_out21, uint32_t *d_out2N,
                                      size_t count, cudaStream_t s, uint32_t *d_part)
 {
@@ -808,11 +808,11 @@ extern "C" int luthe_check_device_error(luthe_ctx *c)
         cudaMemset(c->d_err, 0, 4);
         if (e & DEVERR_DRAIN)
             return fail(LUTHE_E_TIMEOUT,
-                        "blind rotation: a bounded wait ran out and a BSK copy still in flight did not finish "
-                        "landing in shared memory; the device state is unsafe: destroy this context and "
+                        "blind rotation or key switch: a bounded wait ran out and a copy or product still in flight "
+                        "did not finish in time; the device state is unsafe: destroy this context and "
                         "end the process before further use of the device");
         if (e & DEVERR_TIMEOUT)
-            return fail(LUTHE_E_TIMEOUT, "blind rotation: bounded wait for a BSK slab ran out%s",
+            return fail(LUTHE_E_TIMEOUT, "blind rotation or key switch: a bounded wait ran out%s",
                         (e & DEVERR_LUT_ID) ? " (and a LUT id was out of range)" : "");
         return fail(LUTHE_E_PARAM, "blind rotation: a LUT id was >= the uploaded LUT count (%u)", c->nlut);
     }

@@ -38,7 +38,9 @@
 // the last step, accumulate, rotate, decompose, forward transform), then
 // product units (tile of 128 ciphertexts, point, column).  CTAs meet through
 // counters per tile, not through a barrier.  What they exchange (64 KiB per
-// ciphertext and step) and the accumulators stay in L2.
+// ciphertext and step) and the accumulators stay in L2 up to about 300
+// ciphertexts; a launch of 592 writes 18 KB per ciphertext and step of it back
+// to memory (ncu, 64 steps: 676 MB, 296 ciphertexts 5 MB).
 //
 // Reference steps: hw/module/pe_pbs feed_rot.sv:305-307, feed_final.sv:324,
 // decomp_balseq_core.sv:135-150, ntt_core_gf64, pp_core,

@@ -189,8 +189,10 @@ cudaError_t launch_ntt_mul(const uint64_t *d_a, const uint64_t *d_b, uint64_t *d
 // halves (rows 4g, 4g+1 and 4g+2, 4g+3).  One dp4a multiplies the four low
 // bytes by four packed digits (signed bytes) and two dp2a the upper parts:
 // three instructions replace four 32-bit multiply-adds, with two
-// accumulators per output.  Templated
-// on the decomposition (base 2^BL, L levels) of the reference's parameter sets.
+// accumulators per output.  Templated on the decomposition (base 2^BL, L
+// levels) of the reference's parameter sets.  Runs in contexts without room
+// for the tensor-core form (ks_tc.cu) and in the serving lanes.
+
 // acc + sum over the 4 bytes of (unsigned byte of k) * (signed byte of d)
 __device__ __forceinline__ int dp4a_us(u32 k, u32 d, int acc)
 {

@@ -46,13 +46,13 @@ cudaError_t launch_ntt_mul(const uint64_t *d_a, const uint64_t *d_b, uint64_t *d
 // Tie rule of the balanced decompositions for a top digit equal to B/2:
 // the RTL's (decomp_parallel.sv) or the reference's test-vector generator's.
 constexpr uint32_t TIE_RTL = 0, TIE_GENERATOR = 1;
+// d_part: KS_BM x xpad u32, all zero, for the split-K form of batches of at
+// most KS_BM ciphertexts (left zero again); nullptr: the one-pass form only.
+// Calls that overlap on the GPU must not share it.
 cudaError_t launch_keyswitch(const uint64_t *d_in, const uint32_t *d_ksk_t, uint32_t *d_out21, uint32_t *d_out2N,
                              size_t B, uint32_t n, uint32_t xpad, cudaStream_t s,
                              const uint32_t *d_src_idx = nullptr, uint32_t bl = KS_BL, uint32_t L = KS_L,
                              uint32_t tie_rule = TIE_RTL, uint32_t *d_part = nullptr);
-// d_part: KS_BM x xpad u32, all zero, for the split-K form of batches of at
-// most KS_BM ciphertexts (left zero again); nullptr: the one-pass form only.
-// Calls that overlap on the GPU must not share it.
 // The split-K forms' epilogue: outputs of the partial sums, which are cleared.
 cudaError_t launch_ks_finish(const uint64_t *d_in, uint32_t *d_part, uint32_t *d_out21, uint32_t *d_out2N, uint32_t B,
                              uint32_t n, uint32_t xpad, cudaStream_t s);
@@ -106,9 +106,9 @@ enum LweOp : int { LWE_ADD = 0, LWE_SUB = 1, LWE_MAC = 2, LWE_ADDS = 3, LWE_SUBS
 // one linear DOp or register copy (op = LWE_COPY) on slots of a BLWE pool
 constexpr int LWE_COPY = 7;
 // device error flag bits (luthe_check_device_error)
-constexpr uint32_t DEVERR_TIMEOUT = 1u;  // a bounded wait for a BSK slab ran out
+constexpr uint32_t DEVERR_TIMEOUT = 1u;  // a bounded wait ran out
 constexpr uint32_t DEVERR_LUT_ID = 2u;   // a LUT id >= the uploaded LUT count
-constexpr uint32_t DEVERR_DRAIN = 4u;    // after a timeout, a slab copy in flight did not finish landing
+constexpr uint32_t DEVERR_DRAIN = 4u;    // after a timeout, copies or products in flight did not finish in time
 struct AluOp {
     uint32_t op, dst, a, b;
     uint64_t imm;

@@ -16,10 +16,10 @@
 // and add their partial sums into a buffer (32-bit wrap-around sums are exact
 // mod 2^21 in any order).
 //
-// One B200, n = 804, KS 3x6: 16384 BLWEs in 0.54 ms against 10.35 ms with
+// One B200, n = 804, KS 3x6: 16384 BLWEs in 0.55 ms against 10.35 ms with
 // dp4a/dp2a on the multiply pipe (per pass of 3584: digits 26 us, product 91 us,
 // 450 clocks per K step where L2 would allow 390 and the MMAs 256), 65 BLWEs of
-// the 2x7 set 27 us against 1.27 ms.
+// the 2x7 set 24.6 us against 1.24 ms.
 #include <algorithm>
 
 #include "kernels.cuh"
