@@ -35,8 +35,7 @@ def _deps():
 def build_engine(force=False, verbose=False):
     if not force and _newer(LIB, _deps()):
         return LIB
-    # host functions at 32-byte boundaries: the key generation's loops take 14 % longer at odd multiples of 16
-    cmd = [NVCC, *ARCH, "-O3", "-lineinfo", "-std=c++17", "-shared", "-Xcompiler", "-fPIC,-fopenmp,-falign-functions=32",
+    cmd = [NVCC, *ARCH, "-O3", "-lineinfo", "-std=c++17", "-shared", "-Xcompiler", "-fPIC,-fopenmp",
            "-I", os.path.join(ROOT, "include"), "-o", LIB]
     if verbose:
         cmd += ["-Xptxas", "-v"]
