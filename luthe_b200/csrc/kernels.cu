@@ -1163,6 +1163,7 @@ cudaError_t launch_blind_rotate(const BrConfig &cfg, int nsm, const uint32_t *d_
     if (tie_rule != TIE_RTL && tie_rule != TIE_GENERATOR) return cudaErrorInvalidValue;
     const int G = cfg.cts_per_cta, cps = cfg.ctas_per_sm;
     const size_t wave = (size_t)nsm * cps * G;
+    const size_t pair_max = cfg.pair_max >= 0 ? (size_t)cfg.pair_max : (size_t)(nsm / 2);
     const size_t split_max = cfg.split_max >= 0 ? (size_t)cfg.split_max : (size_t)nsm;
     const size_t tail_max = cfg.tail_max >= 0 ? (size_t)cfg.tail_max : (size_t)nsm;
     // A batch that fits one ciphertext per SM runs in the latency form (one
@@ -1174,7 +1175,10 @@ cudaError_t launch_blind_rotate(const BrConfig &cfg, int nsm, const uint32_t *d_
     // As many as fit at the same time go on clusters of eight or four SMs (15 and
     // 33 on 148 SMs: 3.0 and 4.3 ms against 6.8 ms of the two-SM form; the 16th
     // would wait for a whole bootstrap, 6.0 ms).
-    auto small_form = [&](size_t count) { return -(br_small_sms(cfg, nsm, count) / 2); };
+    auto small_form = [&](size_t count) {
+        if (count > pair_max) return 0;
+        return count <= (size_t)cfg.oct_max ? -4 : count <= (size_t)cfg.quad_max ? -2 : -1;
+    };
     if (G > 1 && B <= split_max)
         return launch_br_once(small_form(B), 1, nsm, d_lwe2N, d_luts, d_lut_id, nlut, d_bsk, d_tw, d_out, B, n,
                               d_err, s, d_dst_idx, mlk, pbs_bw, tie_rule);

@@ -92,12 +92,6 @@ cudaError_t launch_blind_rotate(const BrConfig &cfg, int num_sms, const uint32_t
                                 const uint32_t *d_dst_idx = nullptr, uint32_t mlk = 1, uint32_t pbs_bw = 23,
                                 uint32_t tie_rule = TIE_RTL, cudaEvent_t main_done = nullptr,
                                 size_t *main_count = nullptr);
-// SMs that each ciphertext of a small batch runs on (launch_blind_rotate)
-inline int br_small_sms(const BrConfig &cfg, int num_sms, size_t count)
-{
-    if (count > (cfg.pair_max >= 0 ? (size_t)cfg.pair_max : (size_t)(num_sms / 2))) return 1;
-    return count <= (size_t)cfg.oct_max ? 8 : count <= (size_t)cfg.quad_max ? 4 : 2;
-}
 size_t br_smem_bytes(const BrConfig &cfg, uint32_t n);
 cudaError_t br_set_attributes(const BrConfig &cfg, uint32_t n);
 void br_cluster_limits(BrConfig *cfg);  // sets oct_max and quad_max for the current device

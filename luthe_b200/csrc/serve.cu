@@ -239,7 +239,6 @@ struct Lane {
     uint32_t *d_part = nullptr;  // split-K partial sums of this lane's small key switches (kept zero)
     uint32_t *h_idx = nullptr;   // pinned staging of d_idx
     std::vector<std::pair<Request *, int>> ops;
-    int sms = 0;                 // SMs to a ciphertext of the batch in flight
     bool busy = false;
 };
 
@@ -566,24 +565,17 @@ extern "C" int luthe_server_step(luthe_server *s, uint32_t *n_completed, uint32_
         }
         // Clusters hold eight, four or two SMs per ciphertext for 3.0, 4.3 or
         // 6.9 ms.  When the ciphertexts already on the GPU and this batch
-        // would need more SMs than there are, or more clusters than fit (a
-        // cluster stays within a GPC: 15 of eight SMs and 33 of four on 148),
-        // clusters would queue, the last ones for a whole bootstrap; the batch
-        // then takes the next smaller cluster, in the end one ciphertext per
-        // CTA (10.4 ms on one SM: about 40 % more bootstraps per SM-second
-        // than pairs).  One in flight on eight SMs takes the place of two
-        // clusters of four.
-        size_t inflight = 0, octs = 0;
+        // would need more SMs than there are, clusters would queue for SMs;
+        // the batch then takes the next smaller cluster, in the end one
+        // ciphertext per CTA (10.4 ms on one SM: about 40 % more bootstraps
+        // per SM-second than pairs).
+        size_t inflight = 0;
         for (const Lane &o : s->lanes)
-            if (o.busy) {
-                inflight += o.ops.size();
-                if (o.sms == 8) octs += o.ops.size();
-            }
+            if (o.busy) inflight += o.ops.size();
         BrConfig cfg = c->br;
-        if (8 * (inflight + B) > (size_t)c->nsm || inflight + B > (size_t)cfg.oct_max) cfg.oct_max = 0;
-        if (4 * (inflight + octs + B) > (size_t)c->nsm || inflight + octs + B > (size_t)cfg.quad_max) cfg.quad_max = 0;
+        if (8 * (inflight + B) > (size_t)c->nsm) cfg.oct_max = 0;
+        if (4 * (inflight + B) > (size_t)c->nsm) cfg.quad_max = 0;
         if (2 * (inflight + B) > (size_t)c->nsm) cfg.pair_max = 0;
-        ln.sms = cfg.cts_per_cta > 1 ? br_small_sms(cfg, c->nsm, B) : 1;
         CUDA_TRY(cudaStreamWaitEvent(ln.stream, s->alu_done, 0));
         CUDA_TRY(cudaMemcpyAsync(ln.d_idx, ln.h_idx, (size_t)s->max_pbs * 3 * 4, cudaMemcpyHostToDevice, ln.stream));
         CUDA_TRY(launch_keyswitch(s->d_pool, c->d_ksk, nullptr, ln.d_l2n, B, n, c->xpad, ln.stream, ln.d_idx, c->p.ks_base_log, c->p.ks_level, c->tie_rule,

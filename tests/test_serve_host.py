@@ -36,8 +36,6 @@ def H():
     lib.harness_set_nsm.argtypes = [vp, ctypes.c_int]
     lib.harness_launch_log.argtypes = [vp, vp, ctypes.c_int]
     lib.harness_launch_log.restype = ctypes.c_int
-    lib.harness_set_clusters.argtypes = [vp, ctypes.c_int, ctypes.c_int]
-    lib.harness_cluster_log.argtypes = [vp, vp, ctypes.c_int]
     return lib
 
 
@@ -225,36 +223,3 @@ def test_loaded_gpu_runs_small_batches_one_per_cta(H):
     assert np.all(pair_max[2 * batch > 8] == 0)             # alone too big for the pairs
     assert np.any((pair_max == 0) & (2 * batch <= 8))       # too big with the busy lanes' ciphertexts
     assert np.any(pair_max == -1)                           # room left: the default cut-off
-
-
-@pytest.mark.parametrize("batches,sms", [
-    ([10, 5, 1, 2, 1], [8, 8, 4, 4, 2]),          # 15 fit on clusters of eight; two of four SMs in one of eight
-    ([16, 17, 1], [4, 4, 2]),                     # 33 on clusters of four
-    ([15, 4, 30], [8, 2, 2]),                     # 4 would need the 31st to 34th cluster of four
-    ([33, 1, 41], [4, 2, 1]),                     # 75 pairs do not fit
-])
-def test_batches_take_clusters_that_are_free(H, batches, sms):
-    """A batch runs on clusters of eight or four SMs only while these, as many as
-    the device holds at once (15 and 33 here), have room for it beside the
-    batches in flight; every lane stays busy."""
-    s = PlainServer(H, 1 << 15)
-    H.harness_set_clusters(s.ctx, 15, 33)
-    H.harness_set_nsm(s.ctx, 148)
-    H.harness_launch_log(None, None, 0)
-    H.harness_set_event_lag(1 << 30)
-    try:
-        for m in batches:
-            p = I.Program(m, m)
-            for k in range(m):
-                p.ld(k, k)
-                p.pbs(64 + k, k, "MsgOnly")
-                p.st(k, 64 + k)
-            assert s.submit(p.array(), [1] * m, m)[0] == 0
-            s.step()
-        got = np.zeros(16, np.int32)
-        n = H.harness_cluster_log(s.ctx, got.ctypes.data, 16)
-    finally:
-        H.harness_set_event_lag(0)
-    H.harness_launch_log(None, None, 0)
-    s.close()
-    assert got[:n].tolist() == sms
