@@ -64,12 +64,14 @@ cudaError_t launch_keyswitch(const uint64_t *in, const uint32_t *, uint32_t *, u
 }
 // launches seen: batch size and the cluster-pair cut-off the scheduler passed
 static std::vector<std::pair<size_t, int>> g_launch_log;
+static std::vector<BrConfig> g_config_log;  // and all of its cut-offs
 cudaError_t launch_blind_rotate(const BrConfig &cfg, int, const uint32_t *l2n, const uint64_t *luts, const uint32_t *ids,
                                 uint32_t, const uint64_t *, const uint64_t *, uint64_t *out, size_t B, uint32_t n,
                                 uint32_t *, cudaStream_t, const uint32_t *dst_idx, uint32_t mlk, uint32_t, uint32_t,
                                 cudaEvent_t, size_t *)
 {
     g_launch_log.push_back({B, cfg.pair_max});
+    g_config_log.push_back(cfg);
     for (size_t c = 0; c < B; c++) {
         const uint32_t x = l2n[c * (n + 1)];
         if (x >= 16 / mlk) return cudaErrorInvalidValue;  // payload out of the LUT's range
@@ -105,6 +107,24 @@ extern "C" int harness_launch_log(int64_t *batch, int *pair_max, int cap)
         pair_max[i] = luthe::g_launch_log[i].second;
     }
     luthe::g_launch_log.clear();
+    luthe::g_config_log.clear();
+    return n;
+}
+extern "C" void harness_set_clusters(luthe_ctx *c, int oct_max, int quad_max)
+{
+    c->br.oct_max = oct_max;
+    c->br.quad_max = quad_max;
+}
+// SMs per ciphertext that the logged launches run on (before harness_launch_log clears the log)
+extern "C" int harness_cluster_log(luthe_ctx *c, int *sms, int cap)
+{
+    const int n = (int)luthe::g_config_log.size();
+    for (int i = 0; i < n && i < cap; i++) {
+        const BrConfig &b = luthe::g_config_log[i];
+        const size_t count = luthe::g_launch_log[i].first;
+        const size_t pair_max = b.pair_max >= 0 ? (size_t)b.pair_max : (size_t)(c->nsm / 2);
+        sms[i] = count > pair_max ? 1 : count <= (size_t)b.oct_max ? 8 : count <= (size_t)b.quad_max ? 4 : 2;
+    }
     return n;
 }
 

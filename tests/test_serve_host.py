@@ -36,6 +36,8 @@ def H():
     lib.harness_set_nsm.argtypes = [vp, ctypes.c_int]
     lib.harness_launch_log.argtypes = [vp, vp, ctypes.c_int]
     lib.harness_launch_log.restype = ctypes.c_int
+    lib.harness_set_clusters.argtypes = [vp, ctypes.c_int, ctypes.c_int]
+    lib.harness_cluster_log.argtypes = [vp, vp, ctypes.c_int]
     return lib
 
 
@@ -223,3 +225,35 @@ def test_loaded_gpu_runs_small_batches_one_per_cta(H):
     assert np.all(pair_max[2 * batch > 8] == 0)             # alone too big for the pairs
     assert np.any((pair_max == 0) & (2 * batch <= 8))       # too big with the busy lanes' ciphertexts
     assert np.any(pair_max == -1)                           # room left: the default cut-off
+
+
+@pytest.mark.parametrize("batches,sms", [
+    ([15, 3, 1], [8, 8, 4]),      # 18 ciphertexts are 144 SMs of eight each
+    ([16, 21, 1], [4, 4, 2]),     # 16 do not fit on clusters of eight at once; 37 are 148 SMs of four each
+    ([34, 3, 37, 1], [2, 4, 2, 1]),
+])
+def test_batches_take_the_largest_clusters_the_SMs_allow(H, batches, sms):
+    """The cluster form of each batch beside those in flight: no larger than fits
+    the batch alone (15 clusters of eight SMs, 33 of four), and no more SMs in
+    all than there are.  Every lane stays busy."""
+    s = PlainServer(H, 1 << 15)
+    H.harness_set_clusters(s.ctx, 15, 33)
+    H.harness_set_nsm(s.ctx, 148)
+    H.harness_launch_log(None, None, 0)
+    H.harness_set_event_lag(1 << 30)
+    try:
+        for m in batches:
+            p = I.Program(m, m)
+            for k in range(m):
+                p.ld(k, k)
+                p.pbs(64 + k, k, "MsgOnly")
+                p.st(k, 64 + k)
+            assert s.submit(p.array(), [1] * m, m)[0] == 0
+            s.step()
+        got = np.zeros(16, np.int32)
+        n = H.harness_cluster_log(s.ctx, got.ctypes.data, 16)
+    finally:
+        H.harness_set_event_lag(0)
+    H.harness_launch_log(None, None, 0)
+    s.close()
+    assert got[:n].tolist() == sms
