@@ -24,8 +24,9 @@
  *    the tensor-core forms (blind rotations above one ciphertext per SM, key
  *    switches) need no order: calls that use them wait for one another on the
  *    GPU.  Launches captured by the caller use a second set of them, which the
- *    context's own calls leave alone; replays of such launches of one context
- *    must not overlap each other.
+ *    context's own calls leave alone (without room for it in the budget they
+ *    run the other forms); replays of such launches of one context must not
+ *    overlap each other.
  *
  * Data formats (u64 torus values mod 2^64 unless stated)
  *  - BLWE: N mask coefficients in natural order, then the body
@@ -41,8 +42,8 @@
  *    it to its own evaluation layout on upload (the HPU too receives its BSK
  *    pre-transformed from the host: hw/module/bsk/module/bsk_manager), and,
  *    where the HBM budget has room for it, to the operand form of the
- *    tensor-core blind rotation (2.0 MB per LWE coefficient and two workspaces
- *    of 63 MB; given up again when a later allocation needs the room, but for
+ *    tensor-core blind rotation (2.0 MB per LWE coefficient and one or two
+ *    workspaces of 63 MB; given up again when a later allocation needs the room, but for
  *    forms that launches captured by the caller use: those stay until the
  *    context ends and no longer count against the budget).
  *  - LUT:  trivial GLWE, mask polynomial then body polynomial, natural order.

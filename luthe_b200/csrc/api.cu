@@ -56,7 +56,6 @@ static int check_params(const luthe_params *p)
     return LUTHE_OK;
 }
 
-static size_t brx_bytes(const luthe_ctx *c);
 static void brx_release(luthe_ctx *c);
 static void kstc_release(luthe_ctx *c);
 
@@ -65,7 +64,7 @@ static void kstc_release(luthe_ctx *c);
 // budget, which would otherwise refuse what they used to give way to.
 static size_t held_bytes(const luthe_ctx *c)
 {
-    return (c->ws_held ? brx_bytes(c) : 0) + (c->kt_held ? c->kt_bytes : 0);
+    return (c->ws_held ? c->ws_bytes : 0) + (c->kt_held ? c->kt_bytes : 0);
 }
 static bool over_budget(const luthe_ctx *c, size_t bytes) { return c->used - held_bytes(c) + bytes > c->budget; }
 
@@ -105,10 +104,10 @@ void drop_graphs(luthe_ctx *c)
 
 // ---- tensor-core blind rotation: expanded key and workspace (brx.cu)
 
-static size_t brx_bytes(const luthe_ctx *c)
+static size_t brx_bytes(const luthe_ctx *c, int sets)
 {
     using namespace brx;
-    return (size_t)c->p.lwe_dim * STEP_BYTES + WEIGHT_BYTES + 2 * BUFFER_BYTES;
+    return (size_t)c->p.lwe_dim * STEP_BYTES + WEIGHT_BYTES + sets * BUFFER_BYTES;
 }
 
 static void brx_release(luthe_ctx *c)
@@ -117,17 +116,20 @@ static void brx_release(luthe_ctx *c)
     drop_graphs(c);  // captured launches use the workspace
     cudaFree(c->ws.weights);  // one allocation
     c->ws = c->ws_cap = brx::Workspace{};
-    c->used -= brx_bytes(c);
+    c->used -= c->ws_bytes;
+    c->ws_bytes = 0;
 }
 
 // Allocate (first key) and fill the expanded key from the standard-domain BSK
 // on the device.  Where it has no room or cannot be set up the context works
-// without: every batch then runs the butterfly kernels.
+// without: every batch then runs the butterfly kernels.  With room for one set
+// of buffers only, launches that the caller captures do.
 static int brx_prepare(luthe_ctx *c, const uint64_t *d_std)
 {
     using namespace brx;
     if (!c->ws.weights) {
-        const size_t bytes = brx_bytes(c);
+        const int sets = over_budget(c, brx_bytes(c, 2)) ? 1 : 2;
+        const size_t bytes = brx_bytes(c, sets);
         int cooperative = 0;
         CUDA_TRY(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, c->device));
         if (!cooperative || over_budget(c, bytes)) return LUTHE_OK;
@@ -138,7 +140,7 @@ static int brx_prepare(luthe_ctx *c, const uint64_t *d_std)
         }
         Workspace w[2];
         cudaError_t e = cudaSuccess;
-        for (int k = 0; k < 2 && e == cudaSuccess; k++) {
+        for (int k = 0; k < sets && e == cudaSuccess; k++) {
             w[k].weights = base;
             w[k].bsk = base + WEIGHT_BYTES;
             w[k].eval = (uint64_t *)(w[k].bsk + (size_t)c->p.lwe_dim * STEP_BYTES + k * BUFFER_BYTES);
@@ -159,6 +161,7 @@ static int brx_prepare(luthe_ctx *c, const uint64_t *d_std)
         }
         c->ws = w[0];
         c->ws_cap = w[1];
+        c->ws_bytes = bytes;
         c->used += bytes;
     }
     CUDA_TRY(launch_expand(d_std, c->ws, c->p.lwe_dim, 0));
@@ -180,27 +183,30 @@ static void kstc_release(luthe_ctx *c)
 // Allocate (first key) and fill the key's form from the KSK as uploaded (d_raw,
 // on the device).  Without room, or where it cannot be set up, every key switch
 // runs the dp4a form.  The digit buffer holds 14 row tiles of 256 (140 product
-// CTAs at ten column tiles, one wave), less where the budget is short.
+// CTAs at ten column tiles, one wave), less where the budget is short of one
+// set of buffers; without the second, captured launches run the dp4a form.
 static int kstc_prepare(luthe_ctx *c, const uint32_t *d_raw)
 {
     const uint32_t n = c->p.lwe_dim, L = c->p.ks_level;
     if (!c->kt.ksk) {
         const size_t ksk = kstc_ksk_bytes(n, L), part = KSTC_PART_ROWS * (size_t)c->xpad * 4;
         size_t rows = 3584;
-        while (rows >= 256 && over_budget(c, ksk + 2 * (part + kstc_digit_bytes(rows, L)))) rows /= 2;
+        while (rows >= 256 && over_budget(c, ksk + part + kstc_digit_bytes(rows, L))) rows /= 2;
         if (rows < 256) return LUTHE_OK;
-        const size_t set = part + kstc_digit_bytes(rows, L), bytes = ksk + 2 * set;
+        const size_t set = part + kstc_digit_bytes(rows, L);
+        const bool two = !over_budget(c, ksk + 2 * set);
+        const size_t bytes = ksk + (two ? 2 : 1) * set;
         uint8_t *base = nullptr;
         if (cudaMalloc((void **)&base, bytes) != cudaSuccess) {
             cudaGetLastError();
             return LUTHE_OK;
         }
         c->kt = KsTc{base, base + ksk + part, (uint32_t *)(base + ksk), rows};
-        c->kt_cap = KsTc{base, c->kt.dig + set, (uint32_t *)(base + ksk + set), rows};
+        if (two) c->kt_cap = KsTc{base, c->kt.dig + set, (uint32_t *)(base + ksk + set), rows};
         c->kt_bytes = bytes;
         c->used += bytes;
         cudaError_t e = cudaMemset(c->kt.part, 0, part);
-        if (e == cudaSuccess) e = cudaMemset(c->kt_cap.part, 0, part);
+        if (e == cudaSuccess && two) e = cudaMemset(c->kt_cap.part, 0, part);
         if (e == cudaSuccess) e = kstc_set_attributes();
         if (e != cudaSuccess) {
             cudaGetLastError();
@@ -335,7 +341,7 @@ extern "C" int luthe_upload_bsk_eval(luthe_ctx *c, const uint64_t *h)
     // the expanded key is made from the standard domain; it must not outlive the key it was made from, so the
     // memory for that copy comes before any change of the key
     uint64_t *d_std = nullptr;
-    const size_t need = words * 8 + (c->ws.weights ? 0 : brx_bytes(c));
+    const size_t need = words * 8 + (c->ws.weights ? 0 : brx_bytes(c, 1));
     if (c->ws_held) {  // captured launches read it: it has to follow the key
         CUDA_TRY(cudaMalloc((void **)&d_std, words * 8));
         c->used += words * 8;
@@ -504,12 +510,12 @@ static cudaError_t enqueue_blind_rotate(luthe_ctx *c, const uint32_t *d_l2n, con
     const bool limited = brx::limited_stream(s);
     BrConfig cfg = c->br;
     if (limited) cfg.oct_max = cfg.quad_max = 0;
-    if (!c->ws.bsk || count <= (size_t)c->nsm || limited)
+    const Run run = run_of(c, s);
+    const brx::Workspace &ws = run == Run::CALLER ? c->ws_cap : c->ws;
+    if (!ws.bsk || count <= (size_t)c->nsm || limited)
         return launch_blind_rotate(cfg, c->nsm, d_l2n, c->d_luts, d_ids, c->nlut, c->d_bsk, c->d_tw, d_out, count, n,
                                    c->d_err, s, nullptr, mlk, c->p.pbs_base_log, c->tie_rule, main_done, main_count);
     if (main_count) *main_count = count;
-    const Run run = run_of(c, s);
-    const brx::Workspace &ws = run == Run::CALLER ? c->ws_cap : c->ws;
     auto launches = [&]() -> cudaError_t {
         for (size_t done = 0; done < count;) {
             const size_t left = count - done, take = std::min(left, brx::WAVE);
@@ -546,10 +552,11 @@ static cudaError_t enqueue_blind_rotate(luthe_ctx *c, const uint32_t *d_l2n, con
 static cudaError_t enqueue_keyswitch(luthe_ctx *c, const uint64_t *d_in, uint32_t *d_out21, uint32_t *d_out2N,
                                      size_t count, cudaStream_t s, uint32_t *d_part)
 {
-    if (c->kt.ksk) {
-        const Run run = run_of(c, s);
+    const Run run = run_of(c, s);
+    const KsTc &kt = run == Run::CALLER ? c->kt_cap : c->kt;
+    if (kt.ksk) {
         auto launches = [&] {
-            return launch_keyswitch_tc(run == Run::CALLER ? c->kt_cap : c->kt, c->nsm, d_in, d_out21, d_out2N, count,
+            return launch_keyswitch_tc(kt, c->nsm, d_in, d_out21, d_out2N, count,
                                        c->p.lwe_dim, c->xpad, c->p.ks_base_log, c->p.ks_level, c->tie_rule, c->d_err, s);
         };
         if (run == Run::NOW) return in_turn(c->kt_done, s, launches);

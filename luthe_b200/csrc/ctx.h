@@ -41,12 +41,13 @@ struct luthe_ctx {
     luthe::BrConfig br{2, 1};
     uint32_t tie_rule = luthe::TIE_RTL;  // decomposition tie rule (luthe_set_tie_rule)
     // tensor-core blind rotation (ws.bsk null: not available) and key switch (kt.ksk null): the keys, and two sets of
-    // buffers, for the context's calls, which take turns at them whatever streams they run on (ws_done, kt_done: the
-    // last one's work), and for launches that the caller captures, whose replays the context does not see
+    // buffers: one for the context's calls, which take turns at it whatever streams they run on (ws_done, kt_done: the
+    // last one's work), and, where there is room, one for launches that the caller captures, whose replays the context
+    // does not see (without it they run the other forms)
     luthe::brx::Workspace ws, ws_cap;
     luthe::KsTc kt, kt_cap;
     cudaEvent_t ws_done = nullptr, kt_done = nullptr;
-    size_t kt_bytes = 0;
+    size_t ws_bytes = 0, kt_bytes = 0;
     bool ws_held = false, kt_held = false;  // used by launches that the caller captured
     bool own_capture = false;               // a graph of luthe_ks_pbs_graph is being captured
     std::vector<GraphEntry> graphs;

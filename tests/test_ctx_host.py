@@ -175,3 +175,29 @@ def test_a_refused_cooperative_launch_runs_the_other_form(ctx):
     assert ctx.log() == ["br 592", "br 108"]
     ctx.lib.harness_fail_brx(1)  # any other error is reported
     assert ctx.call("blind_rotate", 700, ctx.lib.harness_stream()) == L.E_CUDA
+
+
+@pytest.mark.parametrize("name,first,direct,captured", [("blind_rotate", "ksk", "brx 300", "br 300"),
+                                                        ("keyswitch", "bsk", "ks_tc 300", "ks_dp4a 300")])
+def test_a_budget_for_one_set_of_buffers(lib, name, first, direct, captured):
+    """A budget that holds a tensor-core form with one set of buffers, not two:
+    the context's calls use it, and captured launches take the other form."""
+    def uploads(c):
+        for key in (first, "ksk" if first == "bsk" else "bsk"):
+            assert (c.upload_ksk() if key == "ksk" else c.upload_bsk(1)) == 0
+        assert c.upload_luts() == 0
+        return c
+    probe = uploads(Ctx(lib, keys=False))
+    full = lib.luthe_device_bytes(probe.h)
+    probe.close()
+    c = uploads(Ctx(lib, keys=False, budget=full - (16 << 20)))
+    s = lib.harness_stream()
+    for _ in range(2):
+        assert c.call(name, 300, None) == 0
+        assert c.log() == [direct]
+        lib.harness_begin_capture(s)
+        assert c.call(name, 300, s) == 0
+        lib.harness_end_capture(s)
+        assert c.log() == [captured]
+    assert lib.luthe_device_bytes(c.h) <= full - (16 << 20)
+    c.close()
