@@ -25,8 +25,8 @@
  *    switches) need no order: calls that use them wait for one another on the
  *    GPU.  Launches captured by the caller use a second set of them, which the
  *    context's own calls leave alone (without room for it in the budget they
- *    run the other forms); replays of such launches of one context must not
- *    overlap each other.
+ *    run the other forms); replays of several such graphs of one context must
+ *    not overlap each other.
  *
  * Data formats (u64 torus values mod 2^64 unless stated)
  *  - BLWE: N mask coefficients in natural order, then the body

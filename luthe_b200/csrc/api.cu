@@ -247,8 +247,8 @@ extern "C" int luthe_ctx_create(const luthe_params *p, int device, uint64_t budg
     if (e == cudaSuccess) e = br_set_attributes(BrConfig{1, 1}, p->lwe_dim);
     if (e == cudaSuccess) e = br_set_attributes(BrConfig{2, 1}, p->lwe_dim);
     if (e == cudaSuccess) br_cluster_limits(&c->br);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ws_done, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->kt_done, cudaEventDisableTiming);
+    for (Turn *t : {&c->ws_turn, &c->ws_cap_turn, &c->kt_turn, &c->kt_cap_turn})
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&t->done, cudaEventDisableTiming);
     if (e == cudaSuccess) {
         // diagnostics: LUTHE_SLAB_WAIT_POLLS bounds each BSK-slab wait (0: run out at once)
         const char *polls = getenv("LUTHE_SLAB_WAIT_POLLS");
@@ -287,8 +287,8 @@ extern "C" void luthe_ctx_destroy(luthe_ctx *c)
     dfree(c, c->d_hids, c->hcap * 4);
     if (c->ev_main) cudaEventDestroy(c->ev_main);
     if (c->ev_in) cudaEventDestroy(c->ev_in);
-    if (c->ws_done) cudaEventDestroy(c->ws_done);
-    if (c->kt_done) cudaEventDestroy(c->kt_done);
+    for (Turn *t : {&c->ws_turn, &c->ws_cap_turn, &c->kt_turn, &c->kt_cap_turn})
+        if (t->done) cudaEventDestroy(t->done);
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
     delete c;
 }
@@ -469,26 +469,32 @@ int need_keys(luthe_ctx *c)
 // who may replay it whenever they like: what it uses is held, and its buffers
 // are those of captured launches.  OWN: captured by luthe_ks_pbs_graph; the
 // context drops its graphs with what they use, and their launches take turns.
-enum class Run { NOW, OWN, CALLER };
+struct Run {
+    enum { NOW, OWN, CALLER } by = NOW;
+    unsigned long long capture = 0;
+};
 static Run run_of(luthe_ctx *c, cudaStream_t s)
 {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+    unsigned long long id = 0;
+    if (cudaStreamGetCaptureInfo(s, &st, &id) != cudaSuccess) {
         cudaGetLastError();  // the launch itself reports it
-        return Run::NOW;
+        return Run{};
     }
-    return st != cudaStreamCaptureStatusActive ? Run::NOW : c->own_capture ? Run::OWN : Run::CALLER;
+    return st != cudaStreamCaptureStatusActive ? Run{} : c->own_capture ? Run{Run::OWN, id} : Run{Run::CALLER, id};
 }
-// What `enqueue` puts on stream s runs after the last work that `done` was
-// recorded behind, and `done` then stands for it: streams that the caller left
-// unordered cannot meet in the buffers.  (One context, one thread: luthe.h.)
+// What `enqueue` puts on stream s runs after the last work that had the turn,
+// outside of captures or within one, and then has it itself: streams that the
+// caller left unordered cannot meet in the buffers.  (One context, one thread:
+// luthe.h.)
 template <typename F>
-static cudaError_t in_turn(cudaEvent_t done, cudaStream_t s, F enqueue)
+static cudaError_t in_turn(Turn &t, unsigned long long capture, cudaStream_t s, F enqueue)
 {
-    cudaError_t e = cudaStreamWaitEvent(s, done, 0);
+    cudaError_t e = t.capture == capture ? cudaStreamWaitEvent(s, t.done, 0) : cudaSuccess;
     if (e != cudaSuccess) return e;
     e = enqueue();
-    const cudaError_t r = cudaEventRecord(done, s);  // after an error too: part of the work may run
+    const cudaError_t r = cudaEventRecord(t.done, s);  // after an error too: part of the work may run
+    t.capture = capture;
     return e != cudaSuccess ? e : r;
 }
 
@@ -511,7 +517,7 @@ static cudaError_t enqueue_blind_rotate(luthe_ctx *c, const uint32_t *d_l2n, con
     BrConfig cfg = c->br;
     if (limited) cfg.oct_max = cfg.quad_max = 0;
     const Run run = run_of(c, s);
-    const brx::Workspace &ws = run == Run::CALLER ? c->ws_cap : c->ws;
+    const brx::Workspace &ws = run.by == Run::CALLER ? c->ws_cap : c->ws;
     if (!ws.bsk || count <= (size_t)c->nsm || limited)
         return launch_blind_rotate(cfg, c->nsm, d_l2n, c->d_luts, d_ids, c->nlut, c->d_bsk, c->d_tw, d_out, count, n,
                                    c->d_err, s, nullptr, mlk, c->p.pbs_base_log, c->tie_rule, main_done, main_count);
@@ -540,9 +546,9 @@ static cudaError_t enqueue_blind_rotate(luthe_ctx *c, const uint32_t *d_l2n, con
         }
         return cudaSuccess;
     };
-    if (run == Run::NOW) return in_turn(c->ws_done, s, launches);
-    c->ws_held |= run == Run::CALLER;
-    return launches();
+    if (run.by == Run::OWN) return launches();
+    c->ws_held |= run.by == Run::CALLER;
+    return in_turn(run.by == Run::CALLER ? c->ws_cap_turn : c->ws_turn, run.capture, s, launches);
 }
 
 // Key switch of a batch on stream s: on the tensor cores at every size (one
@@ -553,15 +559,15 @@ static cudaError_t enqueue_keyswitch(luthe_ctx *c, const uint64_t *d_in, uint32_
                                      size_t count, cudaStream_t s, uint32_t *d_part)
 {
     const Run run = run_of(c, s);
-    const KsTc &kt = run == Run::CALLER ? c->kt_cap : c->kt;
+    const KsTc &kt = run.by == Run::CALLER ? c->kt_cap : c->kt;
     if (kt.ksk) {
         auto launches = [&] {
             return launch_keyswitch_tc(kt, c->nsm, d_in, d_out21, d_out2N, count,
                                        c->p.lwe_dim, c->xpad, c->p.ks_base_log, c->p.ks_level, c->tie_rule, c->d_err, s);
         };
-        if (run == Run::NOW) return in_turn(c->kt_done, s, launches);
-        c->kt_held |= run == Run::CALLER;
-        return launches();
+        if (run.by == Run::OWN) return launches();
+        c->kt_held |= run.by == Run::CALLER;
+        return in_turn(run.by == Run::CALLER ? c->kt_cap_turn : c->kt_turn, run.capture, s, launches);
     }
     return launch_keyswitch(d_in, c->d_ksk, d_out21, d_out2N, count, c->p.lwe_dim, c->xpad, s, nullptr, c->p.ks_base_log,
                             c->p.ks_level, c->tie_rule, d_part);
@@ -607,9 +613,9 @@ static cudaError_t launch_own_graph(luthe_ctx *c, const GraphEntry &g)
 {
     auto launch = [&] { return cudaGraphLaunch(g.exec, g.stream); };
     auto rotation = [&] {
-        return c->ws.bsk && g.count > (size_t)c->nsm ? in_turn(c->ws_done, g.stream, launch) : launch();
+        return c->ws.bsk && g.count > (size_t)c->nsm ? in_turn(c->ws_turn, 0, g.stream, launch) : launch();
     };
-    return c->kt.ksk ? in_turn(c->kt_done, g.stream, rotation) : rotation();
+    return c->kt.ksk ? in_turn(c->kt_turn, 0, g.stream, rotation) : rotation();
 }
 
 extern "C" int luthe_ks_pbs_graph(luthe_ctx *c, const uint64_t *d_in, const uint32_t *d_ids, uint64_t *d_out,

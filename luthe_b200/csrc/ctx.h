@@ -15,6 +15,12 @@ struct GraphEntry {
     cudaGraphExec_t exec;
 };
 
+// Whose turn it is at a set of buffers: the last work at them
+struct Turn {
+    cudaEvent_t done = nullptr;
+    unsigned long long capture = 0;  // that `done` was recorded in (0: none)
+};
+
 struct luthe_ctx {
     luthe_params p;
     int device = 0;
@@ -41,12 +47,12 @@ struct luthe_ctx {
     luthe::BrConfig br{2, 1};
     uint32_t tie_rule = luthe::TIE_RTL;  // decomposition tie rule (luthe_set_tie_rule)
     // tensor-core blind rotation (ws.bsk null: not available) and key switch (kt.ksk null): the keys, and two sets of
-    // buffers: one for the context's calls, which take turns at it whatever streams they run on (ws_done, kt_done: the
-    // last one's work), and, where there is room, one for launches that the caller captures, whose replays the context
-    // does not see (without it they run the other forms)
+    // buffers: one for the context's calls, which take turns at it whatever streams they run on, and, where there is
+    // room, one for launches that the caller captures, whose replays the context does not see (without it they run the
+    // other forms); the branches of one capture take turns at that
     luthe::brx::Workspace ws, ws_cap;
     luthe::KsTc kt, kt_cap;
-    cudaEvent_t ws_done = nullptr, kt_done = nullptr;
+    Turn ws_turn, ws_cap_turn, kt_turn, kt_cap_turn;
     size_t ws_bytes = 0, kt_bytes = 0;
     bool ws_held = false, kt_held = false;  // used by launches that the caller captured
     bool own_capture = false;               // a graph of luthe_ks_pbs_graph is being captured

@@ -23,6 +23,7 @@ enum {
 };
 struct fake_graph {
     std::vector<const void *> uses;  // buffers of the captured launches
+    std::map<const void *, std::set<int>> ops;
 };
 struct fake_stream {
     std::set<int> before;            // operations ordered before whatever comes next
@@ -32,7 +33,7 @@ struct fake_stream {
 };
 struct fake_event {
     std::set<int> before;
-    bool captured = false;           // recorded during a capture
+    fake_graph *capture = nullptr;   // recorded during a capture
 };
 typedef fake_stream *cudaStream_t;
 typedef fake_event *cudaEvent_t;
@@ -53,7 +54,6 @@ struct FakeCuda {
     int ops = 0;                             // operations enqueued so far
     std::map<const void *, std::set<int>> uses;  // of each shared buffer
     int races = 0;                           // uses of a buffer not ordered after an earlier one
-    std::vector<const void *> captured_uses; // by launches the caller captures
     std::map<int, int> fail_malloc;          // n-th allocation from now -> error
 };
 static FakeCuda g_fake;
@@ -63,14 +63,11 @@ static inline fake_stream *fake_of(cudaStream_t s) { return s ? s : &g_fake.lega
 static inline void fake_use(const void *buf, cudaStream_t s)
 {
     fake_stream *st = fake_of(s);
-    if (st->capture) {
-        st->capture->uses.push_back(buf);
-        if (st->caller) g_fake.captured_uses.push_back(buf);
-        return;
-    }
-    for (int op : g_fake.uses[buf]) g_fake.races += !st->before.count(op);
+    if (st->capture) st->capture->uses.push_back(buf);
+    std::set<int> &uses = st->capture ? st->capture->ops[buf] : g_fake.uses[buf];
+    for (int op : uses) g_fake.races += !st->before.count(op);
     const int op = g_fake.ops++;
-    g_fake.uses[buf].insert(op);
+    uses.insert(op);
     st->before.insert(op);
 }
 
@@ -140,6 +137,11 @@ static inline cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptur
     *st = fake_of(s)->capture ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
     return cudaSuccess;
 }
+static inline cudaError_t cudaStreamGetCaptureInfo(cudaStream_t s, cudaStreamCaptureStatus *st, unsigned long long *id)
+{
+    *id = (unsigned long long)(size_t)fake_of(s)->capture;
+    return cudaStreamIsCapturing(s, st);
+}
 static inline cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned)
 {
     *e = new fake_event;
@@ -159,14 +161,13 @@ static inline cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent
 }
 static inline cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s)
 {
-    e->captured = fake_of(s)->capture != nullptr;
+    e->capture = fake_of(s)->capture;
     e->before = fake_of(s)->before;
     return cudaSuccess;
 }
 static inline cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned)
 {
-    if (fake_of(s)->capture && !e->captured) return cudaErrorStreamCaptureIsolation;
-    if (!fake_of(s)->capture && e->captured) return cudaErrorCapturedEvent;
+    if (fake_of(s)->capture != e->capture) return e->capture ? cudaErrorCapturedEvent : cudaErrorStreamCaptureIsolation;
     fake_of(s)->before.insert(e->before.begin(), e->before.end());
     return cudaSuccess;
 }

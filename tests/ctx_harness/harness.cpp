@@ -101,6 +101,12 @@ void harness_begin_capture(fake_stream *s)  // the caller's
     s->capture = new fake_graph;
     s->caller = true;
 }
+void harness_fork(fake_stream *from, fake_stream *to)  // `to` joins the capture of `from`
+{
+    to->capture = from->capture;
+    to->caller = from->caller;
+    to->before = from->before;
+}
 fake_graph *harness_end_capture(fake_stream *s)
 {
     fake_graph *g = s->capture;
@@ -114,7 +120,6 @@ void harness_reset()
 {
     g_fake.ops = g_fake.races = 0;
     g_fake.uses.clear();
-    g_fake.captured_uses.clear();
     g_fake.fail_malloc.clear();
     g_log.clear();
     g_fail_map = g_fail_ks_attr = g_fail_brx = 0;

@@ -23,6 +23,7 @@ def lib():
     h.harness_begin_capture.argtypes = h.harness_end_capture.argtypes = [vp]
     h.harness_replay.argtypes = [vp, vp]
     h.harness_limit.argtypes = [vp]
+    h.harness_fork.argtypes = [vp, vp]
     h.harness_fail_brx.argtypes = [ctypes.c_int]
     h.harness_fail_malloc.argtypes = [ctypes.c_int, ctypes.c_int]
     h.harness_fail_optional.argtypes = [ctypes.c_int, ctypes.c_int]
@@ -201,3 +202,18 @@ def test_a_budget_for_one_set_of_buffers(lib, name, first, direct, captured):
         assert c.log() == [captured]
     assert lib.luthe_device_bytes(c.h) <= full - (16 << 20)
     c.close()
+
+
+@pytest.mark.parametrize("name", ["keyswitch", "blind_rotate", "ks_pbs_noalloc"])
+def test_branches_of_one_capture_take_turns(ctx, name):
+    """Calls on the branches of one capture share the set of captured launches:
+    no two uses may overlap.  A later capture starts without the earlier one's."""
+    for _ in range(2):
+        a, b = ctx.lib.harness_stream(), ctx.lib.harness_stream()
+        ctx.lib.harness_begin_capture(a)
+        ctx.lib.harness_fork(a, b)
+        for s in (a, b, b, a):
+            assert ctx.call(name, 300, s) == 0
+        ctx.lib.harness_end_capture(b)
+        ctx.lib.harness_end_capture(a)
+    assert ctx.lib.harness_races() == 0

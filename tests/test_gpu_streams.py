@@ -100,3 +100,27 @@ def test_two_contexts(setup):
             eng.check_device_error()
         for job in jobs:
             job.check()
+
+
+@pytest.mark.parametrize("kind", ["blind_rotate", "keyswitch"])
+def test_branches_of_one_capture(setup, kind):
+    import torch
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    jobs = [Job(setup, kind, 40 + k) for k in range(4)]
+    torch.cuda.synchronize()
+    for _ in range(2):  # two captures
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=a):
+            b.wait_stream(a)
+            for k, job in enumerate(jobs):
+                job.run((a, b)[k % 2])
+            a.wait_stream(b)
+        for job in jobs:
+            job.out.zero_()
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+        setup[0].check_device_error()
+        for job in jobs:
+            job.check()
+        del g
