@@ -91,7 +91,8 @@ cudaError_t launch_bsk_prepare(const uint64_t *d_std_p, uint64_t *d_slab, const 
 // 4.9).  The grid is as long as the batch, so that SMs take the next
 // polynomial as they finish one: a persistent grid left the SMs with an uneven
 // number of them (333: 13.9 us, now 10.2; 1000: 25.3, now 20.5).
-// Bound: the integer ALU; 4096 transforms take 74 to 77 us (85 to 87 before), of
+// Bound: the integer ALU (three quarters busy) and the barriers between the four
+// passes; 4096 transforms take 74 to 77 us (85 to 87 before), of
 // which 20 us are the transfers at the copy's rate; 4096 products 219 us (233).
 
 // forward: coefficient order in, evaluation order k out (A_k = A(psi^{2k+1}))
