@@ -1,8 +1,8 @@
 """The launch forms that batches take where the context has no room for the
 tensor-core forms: one and two ciphertexts per CTA in whole waves and with a
 tail, the autotuned shape, the dp4a key switch in one pass and split over K; and
-every form's bounded wait made to run out.  A budget of 17 MB holds a key of 24
-steps and nothing optional."""
+every form's bounded wait made to run out.  A budget of 20 MB holds a key of 90
+steps (two column tiles of the key switch) and nothing optional."""
 import os
 import subprocess
 import sys
@@ -17,7 +17,7 @@ from conftest import from_dev, to_dev
 
 pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-N, STEPS, BUDGET = 2048, 24, 17 << 20
+N, STEPS, BUDGET = 2048, 90, 20 << 20
 
 
 @pytest.fixture(scope="module")
@@ -28,7 +28,7 @@ def setup():
     with L.Engine(p, hbm_budget=BUDGET) as eng:
         eng.upload_keys(keys)
         eng.upload_luts(luts)
-        assert eng.device_bytes < 8 << 20  # no optional form
+        assert eng.device_bytes < 12 << 20  # no optional form
         yield eng, keys, luts, oracle.OracleBsk(keys["bsk"], STEPS, N)
 
 
