@@ -172,7 +172,8 @@ int luthe_ks_pbs_graph(luthe_ctx *ctx, const uint64_t *d_in, const uint32_t *d_l
  * ciphertexts at n = 804) or LUTHE_E_PARAM is returned.  The first call on a
  * device looks up that array's device address; make that first call before
  * any stream capture.  Calls share the array: calls that overlap on the GPU
- * race.  Keys and LUTs come from the context as for luthe_ks_pbs. */
+ * race.  Keys, LUTs and the buffers of the tensor-core forms (allocated with
+ * the keys) come from the context as for luthe_ks_pbs. */
 int luthe_ks_pbs_noalloc(luthe_ctx *ctx, const uint64_t *d_in, const uint32_t *d_lut_id, uint64_t *d_out,
                          size_t count, void *stream);
 
